@@ -209,6 +209,8 @@ int batch_prepare(dfpt_batch* b) {
     b->ks.occupancy(b->sms, c.grid, c.grid_trace, c.grid_simple);
     c.trace_config = b->trace_config;
     c.grid_trace = b->ks.trace_grid(b->trace_config, b->sms);
+    c.packed = true;  // one launch walks every scene's rays
+    for (const auto& st : b->stores) c.packed = c.packed && st->scene.use_pairs == 3;
     b->ctx_shadow = c;
     b->ctx_shadow.pass = &b->pass_shadow;
     return DFPT_OK;

@@ -390,7 +390,7 @@ __device__ __forceinline__ bool mesh_walk(const DevScene& S, int root, int prim,
     // measured 2.4x slower than the threaded walk: every box on a shadow ray is entered and the
     // pending right children overflow the stack.
     if constexpr (V == 5 && !ANY) {
-        if (S.use_pairs == 2) return mesh_walk_pair_compact<ANY, 8>(S, root, prim, oxo, oyo, ozo, dxo, dyo, dzo, h, st);
+        if (S.use_pairs >= 2) return mesh_walk_pair_compact<ANY, 8>(S, root, prim, oxo, oyo, ozo, dxo, dyo, dzo, h, st);
     }
     const SlabRay sr = slab_ray(oxo, oyo, ozo, dxo, dyo, dzo);
     int node = root;
@@ -460,6 +460,9 @@ __device__ __forceinline__ void slab_interval(float ax, float ay, float az, floa
     tmin = jmax3(jmin(t0x, t1x), jmin(t0y, t1y), jmin(t0z, t1z));
 }
 
+// First triangle of a child from its code in a pair record (-1 inner, -2 empty leaf).
+__device__ __forceinline__ int pair_leaf(int code) { return code >= 0 ? -1 : code == (int)0x80000000 ? -2 : ~code; }
+
 // The threaded walk over pair records (DevScene::pairs), with a short stack in shared memory. An
 // entered inner node's record gives both children's boxes in one load. The left child is tested
 // at once (it follows its parent in preorder, with the same closest distance); the right child's
@@ -509,10 +512,11 @@ __device__ __forceinline__ bool mesh_walk_pair(const DevScene& S, int root, int 
         } else {
             const float4* P = S.pairs + 4 * (size_t)cur;
             const float4 p0 = __ldg(P), p1 = __ldg(P + 1), p2 = __ldg(P + 2);
-            const int4 p3 = __ldg(reinterpret_cast<const int4*>(P + 3));
+            const int4 codes = __ldg(reinterpret_cast<const int4*>(P + 3));
+            const int4 p3 = make_int4(pair_leaf(codes.x), pair_leaf(codes.y), codes.z, 0);
             float lmin, lmax, rmin, rmax;
-            slab_interval(p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, sr, lmin, lmax);
-            slab_interval(p1.z, p1.w, p2.x, p2.y, p2.z, p2.w, sr, rmin, rmax);
+            slab_interval(p0.x, p0.y, p2.x, p0.z, p0.w, p2.y, sr, lmin, lmax);
+            slab_interval(p1.x, p1.y, p2.z, p1.z, p1.w, p2.w, sr, rmin, rmax);
             st.nodes++;
             const bool accept_r = box_accepts(rmin, rmax, h.t);
             if (box_accepts(lmin, lmax, h.t)) {
@@ -580,7 +584,7 @@ __device__ __forceinline__ bool mesh_walk_pair(const DevScene& S, int root, int 
 // finished node in the threaded records, so every node is still tested at its preorder position
 // with the closest distance of that moment: the hits equal mesh_walk's at any stack depth. The
 // visit counter can count a node twice after a drop: the threaded continuation re-tests a right
-// child rejected at its parent's step (it is rejected again). Needs DevScene::use_pairs == 2 (no
+// child rejected at its parent's step (it is rejected again). Needs DevScene::use_pairs >= 2 (no
 // empty leaves) and blocks of at most 256 threads.
 template <bool ANY, int K>
 __device__ __forceinline__ bool mesh_walk_pair_compact(const DevScene& S, int root, int prim, float oxo, float oyo, float ozo,
@@ -627,10 +631,11 @@ __device__ __forceinline__ bool mesh_walk_pair_compact(const DevScene& S, int ro
         } else {
             const float4* P = S.pairs + 4 * (size_t)cur;
             const float4 p0 = __ldg(P), p1 = __ldg(P + 1), p2 = __ldg(P + 2);
-            const int4 p3 = __ldg(reinterpret_cast<const int4*>(P + 3));
+            const int4 codes = __ldg(reinterpret_cast<const int4*>(P + 3));
+            const int4 p3 = make_int4(pair_leaf(codes.x), pair_leaf(codes.y), codes.z, 0);
             float lmin, lmax, rmin, rmax;
-            slab_interval(p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, sr, lmin, lmax);
-            slab_interval(p1.z, p1.w, p2.x, p2.y, p2.z, p2.w, sr, rmin, rmax);
+            slab_interval(p0.x, p0.y, p2.x, p0.z, p0.w, p2.y, sr, lmin, lmax);
+            slab_interval(p1.x, p1.y, p2.z, p1.z, p1.w, p2.w, sr, rmin, rmax);
             st.nodes++;
             const bool accept_r = box_accepts(rmin, rmax, h.t);
             if (box_accepts(lmin, lmax, h.t)) {
@@ -688,6 +693,162 @@ __device__ __forceinline__ bool mesh_walk_pair_compact(const DevScene& S, int ro
             }
         }
     }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The packed pair walk (traversal variant 6): what configurations 16 and 17 run when nothing is counted.
+
+// 32 bytes in one load (sm_100 and later); the address a multiple of 32.
+__device__ __forceinline__ void ldg256(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// SlabRay with its terms paired for the packed float instructions: x and y together, z twice.
+struct SlabRay2 {
+    float2 ixy, iz, pxy, pz;
+};
+__device__ __forceinline__ SlabRay2 slab_ray2(float ox, float oy, float oz, float dx, float dy, float dz) {
+    const SlabRay r = slab_ray(ox, oy, oz, dx, dy, dz);
+    return SlabRay2{make_float2(r.ix, r.iy), make_float2(r.iz, r.iz), make_float2(r.px, r.py), make_float2(r.pz, r.pz)};
+}
+// slab() on both halves, each rounded as slab() rounds it.
+__device__ __forceinline__ float2 slab2(float bx, float by, float2 inv, float2 p) {
+#ifdef DFPT_FMA_SLABS
+    return __ffma2_rn(make_float2(bx, by), inv, p);
+#else
+    return __fmul2_rn(__fadd2_rn(make_float2(bx, by), make_float2(-p.x, -p.y)), inv);
+#endif
+}
+__device__ __forceinline__ void slab_interval2(float2 lo, float2 hi, float2 z, float& tmin, float& tmax) {
+    tmax = jmin3(jmax(lo.x, hi.x), jmax(lo.y, hi.y), jmax(z.x, z.y));
+    tmin = jmax3(jmin(lo.x, hi.x), jmin(lo.y, hi.y), jmin(z.x, z.y));
+}
+// box_accepts with the distance it depends on kept apart: key is the entry, or the exit when the
+// interval begins at or behind 0.001.
+__device__ __forceinline__ float box_key(float tmin, float tmax) { return tmin > 0.001f ? tmin : tmax; }
+__device__ __forceinline__ bool key_accepts(float tmin, float tmax, float key, float closest) {
+    return !(tmin > tmax) && key > 0.001f && key < closest;
+}
+
+// Stack entries {code, key} in shared memory, [entry][thread] for blocks of NT threads; entries past
+// DFPT_WALK_STACK go to the thread's local memory (`deep`). A walk holds at most one entry per level
+// of its tree, and trees deeper than DFPT_WALK_DEPTH levels do not take this walk (scene_upload).
+#define DFPT_WALK_STACK 8
+template <int NT>
+__device__ __forceinline__ int2* walk_stack() {
+    __shared__ int2 stk[DFPT_WALK_STACK * NT];
+    return stk + threadIdx.x;
+}
+
+// One mesh over the pair records, in object space. Returns for any-hit queries whether there is a
+// hit; for closest-hit queries it lowers `closest` and sets `best` to the index of the triangle
+// record (-1: none of this mesh is closer).
+//
+// A record gives both children's boxes in two 32-byte loads and six packed FMAs. Both children
+// accepted: one is pushed with its key (see mesh_walk_pair_compact: key < closest is its box test at
+// any later time) and the other entered.
+// Order. The reference visits in preorder, and one of its box tests depends on that: a box that
+// holds the ray's origin is entered only while its exit lies before the closest hit so far. Such
+// boxes form the top of the tree (a box around the origin has such a parent; scene_upload checks
+// that children lie in their parents), and below one the origin lies outside of lies no other.
+// Inside the subtrees that the ray enters from outside, an unvisited box can only hold hits beyond
+// its entry, so their order does not change the closest hit: there (both children's entries ahead of
+// the origin) the nearer child goes first, everywhere else the left one. Of two triangles hit at
+// the same distance - a ray through their shared edge - the one first in preorder is kept, as the
+// reference keeps it. The strict set, whose ids equal the reference's bit for bit, keeps preorder
+// throughout.
+//
+// Shape of the loop: a lane steps through inner nodes until it holds a leaf or is done; the lanes of
+// a warp meet there and test their leaves together. One loop with a branch per node kind, which lets
+// descending lanes run ahead, measured 22.6 ms against 20.9 for a 32-pass 1080p mesh_scene step
+// (any hit 10.5 against 6.9), and a vote per step 24.8 (7.3).
+//
+// What bounds it: instruction issue at the lanes that divergence leaves (the compact pair walk: 75 %
+// of issue slots at 16 lanes per instruction on camera rays, 67 % at 9 on bounce rays) and the
+// load/store pipe (75 % of its wavefronts); hence wide loads, packed FMAs, no counters, the object-
+// space ray kept from primitive to primitive and no overflow logic on the common path. Closest hits
+// of that step 30.2 -> 20.9 ms; its shadow rays, from the threaded walk, 8.1 -> 6.9.
+#ifdef DFPT_STRICT_MATH
+#define DFPT_NEAR_FIRST false
+#else
+#define DFPT_NEAR_FIRST true
+#endif
+template <bool ANY, int NT>
+__device__ __forceinline__ bool pair_walk(const DevScene& S, int root, float ox, float oy, float oz, float dx, float dy, float dz,
+                                          const SlabRay2& sr, float& closest, int& best) {
+    constexpr int DONE = (int)0x80000000;  // no triangle's complement
+    int2* const stk = walk_stack<NT>();
+    int2 deep[DFPT_WALK_DEPTH - DFPT_WALK_STACK];
+    int top = 0;
+    int code;  // the node to visit: an inner node's index, ~(first triangle) of a leaf, or DONE
+    {
+        float4 n0, n1;
+        ldg256(S.nodes + 2 * root, n0, n1);
+        float tmin, tmax;
+        slab_interval2(slab2(n0.x, n0.y, sr.ixy, sr.pxy), slab2(n1.x, n1.y, sr.ixy, sr.pxy), slab2(n0.z, n1.z, sr.iz, sr.pz), tmin, tmax);
+        const int leaf = __float_as_int(n1.w);
+        code = !key_accepts(tmin, tmax, box_key(tmin, tmax), closest) ? DONE : leaf >= 0 ? ~leaf : root;
+    }
+    // The next pending entry (closest hit: the next whose box is still ahead of it).
+    auto pop = [&]() {
+        code = DONE;
+        while (top > 0) {
+            --top;
+            int2 e;
+            if (top < DFPT_WALK_STACK) e = stk[top * NT];
+            else e = deep[top - DFPT_WALK_STACK];
+            if (ANY || __int_as_float(e.y) < closest) {
+                code = e.x;
+                break;
+            }
+        }
+    };
+    while (code != DONE) {
+        while (code >= 0) {
+            float4 a, b, c, e;
+            const float4* P = S.pairs + 4 * (size_t)code;
+            ldg256(P, a, b);
+            ldg256(P + 2, c, e);
+            float lmin, lmax, rmin, rmax;
+            slab_interval2(slab2(a.x, a.y, sr.ixy, sr.pxy), slab2(a.z, a.w, sr.ixy, sr.pxy), slab2(c.x, c.y, sr.iz, sr.pz), lmin, lmax);
+            slab_interval2(slab2(b.x, b.y, sr.ixy, sr.pxy), slab2(b.z, b.w, sr.ixy, sr.pxy), slab2(c.z, c.w, sr.iz, sr.pz), rmin, rmax);
+            const float lkey = box_key(lmin, lmax), rkey = box_key(rmin, rmax);
+            const bool al = key_accepts(lmin, lmax, lkey, closest), ar = key_accepts(rmin, rmax, rkey, closest);
+            const int lc = __float_as_int(e.x), rc = __float_as_int(e.y);
+            code = al ? lc : rc;
+            if (al && ar) {
+                const bool swap = DFPT_NEAR_FIRST && !ANY && rmin > 0.001f && rmin < lmin;
+                const int2 later = swap ? make_int2(lc, __float_as_int(lkey)) : make_int2(rc, __float_as_int(rkey));
+                if (swap) code = rc;
+                if (top < DFPT_WALK_STACK) stk[top * NT] = later;
+                else deep[top - DFPT_WALK_STACK] = later;
+                ++top;
+            } else if (!al && !ar) {
+                pop();
+            }
+        }
+        if (code == DONE) break;
+        for (int k = ~code;; ++k) {
+            const float4 a = __ldg(S.tris + 3 * k);
+            const float4 e0 = __ldg(S.tris + 3 * k + 1);
+            const float4 e1 = __ldg(S.tris + 3 * k + 2);
+            const float t = isect_triangle(ox, oy, oz, dx, dy, dz, a, e0, e1, INF);
+            if constexpr (ANY) {
+                if (t < INF) {
+                    closest = t;
+                    return true;
+                }
+            } else if (t < closest || (t == closest && k < best)) {
+                closest = t;
+                best = k;
+            }
+            if (__float_as_int(e0.w) != 0) break;
+        }
+        pop();
+    }
+    return false;
 }
 
 // Warp-synchronous form of the same walk: every lane keeps its own position in the preorder
@@ -894,12 +1055,10 @@ __device__ Hit trace(const DevScene& S, float ox, float oy, float oz, float dx, 
 // the closest distance the full loop would have. The reachable primitives are collected from
 // the culling BVH, sorted, merged with the unbounded ones, and tested with prim_test. More than
 // DFPT_CULL_CANDIDATES of them (or a deeper tree than the stack) falls back to the full loop.
-template <bool ANY, int V>
-__device__ Hit trace_culled(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz, TraceStats& st) {
-    const float ix = 1.0f / dx, iy = 1.0f / dy, iz = 1.0f / dz;
-    int cand[DFPT_CULL_CANDIDATES];
+// The candidates in ascending order, or -1 when they overflow DFPT_CULL_CANDIDATES (or the stack).
+__device__ __forceinline__ int cull_collect(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz, float ix,
+                                            float iy, float iz, int* cand) {
     int nc = 0;
-    bool overflow = false;
     int stack[DFPT_CULL_STACK];
     int sp = 0;
     int node = 0;
@@ -909,24 +1068,29 @@ __device__ Hit trace_culled(const DevScene& S, float ox, float oy, float oz, flo
             const int l = __float_as_int(a.w), r = __float_as_int(b.w);
             if (l < 0) {
                 for (int k = -l - 1, e = -l - 1 + r; k < e; ++k) {
-                    if (nc == DFPT_CULL_CANDIDATES) { overflow = true; break; }
+                    if (nc == DFPT_CULL_CANDIDATES) return -1;
                     const int p = __ldg(S.cull_prims + k);
                     int j = nc++;
                     while (j > 0 && cand[j - 1] > p) { cand[j] = cand[j - 1]; --j; }
                     cand[j] = p;
                 }
-                if (overflow) break;
             } else {
-                if (sp == DFPT_CULL_STACK) { overflow = true; break; }
+                if (sp == DFPT_CULL_STACK) return -1;
                 stack[sp++] = r;
                 node = l;
                 continue;
             }
         }
-        if (sp == 0) break;
+        if (sp == 0) return nc;
         node = stack[--sp];
     }
-    if (overflow) {
+}
+template <bool ANY, int V>
+__device__ Hit trace_culled(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz, TraceStats& st) {
+    const float ix = 1.0f / dx, iy = 1.0f / dy, iz = 1.0f / dz;
+    int cand[DFPT_CULL_CANDIDATES];
+    const int nc = cull_collect(S, ox, oy, oz, dx, dy, dz, ix, iy, iz, cand);
+    if (nc < 0) {
         // The full loop, with the per-primitive box test (mode 1).
         DevScene flat = S;
         flat.use_culling = 1;
@@ -953,6 +1117,116 @@ __device__ Hit trace_culled(const DevScene& S, float ox, float oy, float oz, flo
             if (box_entry(lo, hi, ox, oy, oz, dx, dy, dz, ix, iy, iz) > h.t) continue;
         }
         if (prim_test<ANY, V>(S, i, ox, oy, oz, dx, dy, dz, h, st)) return h;
+    }
+    return h;
+}
+
+// A ray in the object space of one primitive, kept while the primitives that follow have the same
+// world-to-object matrix (DevScene::prim_walk names the first of each such run; most scenes place
+// their meshes with one matrix).
+struct ObjRay {
+    float ox, oy, oz, dx, dy, dz;
+    SlabRay2 sr;
+    int matrix;  // primitive whose matrix it was made with, -1 none
+    int slabs;   // the same for sr
+};
+
+// prim_test over the packed pair walk.
+template <bool ANY, int NT>
+__device__ __forceinline__ bool prim_test_pairs(const DevScene& S, int i, float ox, float oy, float oz, float dx, float dy, float dz,
+                                                ObjRay& r, Hit& h) {
+    const int4 info = __ldg(S.prim_walk + i);  // {shape type, shape offset, record, first primitive with this matrix}
+    if (info.w != r.matrix) {
+        const float4* W = reinterpret_cast<const float4*>(S.w2o) + (size_t)info.w * 4;
+        const float4 r0 = __ldg(W), r1 = __ldg(W + 1), r2 = __ldg(W + 2);
+        r.ox = r0.x * ox + r0.y * oy + r0.z * oz + r0.w;
+        r.oy = r1.x * ox + r1.y * oy + r1.z * oz + r1.w;
+        r.oz = r2.x * ox + r2.y * oy + r2.z * oz + r2.w;
+        r.dx = r0.x * dx + r0.y * dy + r0.z * dz;
+        r.dy = r1.x * dx + r1.y * dy + r1.z * dz;
+        r.dz = r2.x * dx + r2.y * dy + r2.z * dz;
+        r.matrix = info.w;
+    }
+    float t = INF;
+    if (info.x == DFPT_SHAPE_TRIANGLE_MESH) {
+        if (r.slabs != r.matrix) {
+            r.sr = slab_ray2(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz);
+            r.slabs = r.matrix;
+        }
+        int best = -1;
+        const bool any = pair_walk<ANY, NT>(S, info.z, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.sr, h.t, best);
+        if constexpr (ANY) {
+            if (any) h.prim = i;
+            return any;
+        }
+        if (best >= 0) {
+            h.prim = i;
+            h.shape_type = DFPT_SHAPE_TRIANGLE;
+            h.shape_offset = __float_as_int(__ldg(S.tris + 3 * (size_t)best).w);
+        }
+        return false;
+    } else if (info.x == DFPT_SHAPE_PLANE) {
+        t = isect_plane(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, __ldg(S.plane_a + info.z), __ldg(S.plane_n + info.z), h.t);
+    } else if (info.x == DFPT_SHAPE_SPHERE) {
+        t = isect_sphere(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, __ldg(S.sphere4 + info.z), h.t);
+    } else if (info.x == DFPT_SHAPE_TERRAIN) {
+        t = isect_terrain(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz);
+    } else if (info.x == DFPT_SHAPE_TRIANGLE) {
+        t = isect_triangle(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, __ldg(S.tris + 3 * info.z), __ldg(S.tris + 3 * info.z + 1),
+                           __ldg(S.tris + 3 * info.z + 2), h.t);
+    }
+    if (t < h.t) {
+        h.t = t;
+        h.prim = i;
+        h.shape_type = info.x;
+        h.shape_offset = info.y;
+    }
+    return ANY && h.prim != -1;
+}
+
+// trace / trace_culled over the packed pair walk: the same primitives in the same order.
+template <bool ANY, int NT>
+__device__ __forceinline__ Hit trace_pairs(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz) {
+    Hit h;
+    h.t = INF;
+    h.prim = -1;
+    h.shape_type = -1;
+    h.shape_offset = -1;
+    ObjRay r;
+    r.matrix = r.slabs = -1;
+    const int np = S.primitive_count;
+    if (S.use_culling == 0) {
+        for (int i = 0; i < np; ++i)
+            if (prim_test_pairs<ANY, NT>(S, i, ox, oy, oz, dx, dy, dz, r, h)) break;
+        return h;
+    }
+    const float ix = 1.0f / dx, iy = 1.0f / dy, iz = 1.0f / dz;
+    int cand[DFPT_CULL_CANDIDATES];
+    int nc = S.use_culling == 2 ? cull_collect(S, ox, oy, oz, dx, dy, dz, ix, iy, iz, cand) : -1;
+    // The candidates merged with the unbounded primitives, or (mode 1, too many candidates) every
+    // primitive behind its own box test.
+    const int na = nc >= 0 ? S.always_count : 0;
+    int ia = 0, ic = 0;
+    for (;;) {
+        int i;
+        bool boxed = true;
+        if (nc >= 0) {
+            const int pa = ia < na ? __ldg(S.always + ia) : 0x7FFFFFFF;
+            const int pc = ic < nc ? cand[ic] : 0x7FFFFFFF;
+            boxed = pc < pa;
+            i = boxed ? pc : pa;
+            if (i == 0x7FFFFFFF) break;
+            ic += boxed ? 1 : 0;
+            ia += boxed ? 0 : 1;
+        } else {
+            if (ic >= np) break;
+            i = ic++;
+        }
+        if (boxed) {
+            const float4 lo = __ldg(S.prim_box + 2 * i), hi = __ldg(S.prim_box + 2 * i + 1);
+            if (box_entry(lo, hi, ox, oy, oz, dx, dy, dz, ix, iy, iz) > h.t) continue;
+        }
+        if (prim_test_pairs<ANY, NT>(S, i, ox, oy, oz, dx, dy, dz, r, h)) break;
     }
     return h;
 }
@@ -1091,11 +1365,13 @@ __device__ __forceinline__ Hit trace_s(const DevScene& S, float ox, float oy, fl
 }
 
 // Selects the walk: V 0/1 per-lane (every lane may call it alone), V 2 warp-synchronous (all 32
-// lanes call it; invalid lanes pass valid = false).
+// lanes call it; invalid lanes pass valid = false), V 6 the packed pair walk (blocks of 256; counts nothing).
 template <bool ANY, int V>
 __device__ __forceinline__ Hit trace_v(const DevScene& S, bool valid, float ox, float oy, float oz, float dx, float dy, float dz, TraceStats& st) {
     if constexpr (V == 2) {
         return trace_warp<ANY>(S, valid, ox, oy, oz, dx, dy, dz, st);
+    } else if constexpr (V == 6) {
+        if (valid) return trace_pairs<ANY, 256>(S, ox, oy, oz, dx, dy, dz);
     } else {
         if (valid) return S.use_culling == 2 ? trace_culled<ANY, V>(S, ox, oy, oz, dx, dy, dz, st) : trace<ANY, V>(S, ox, oy, oz, dx, dy, dz, st);
     }

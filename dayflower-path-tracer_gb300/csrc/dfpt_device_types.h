@@ -29,10 +29,14 @@ struct DevScene {
     const float4* nodes;    // 2 per BVH node: {min.xyz, next}, {max.xyz, first triangle or -1}
     const float4* tris;     // 3 per triangle: {a.xyz, triangle offset}, {b-a, last-in-leaf}, {c-a, leaf node index}
     const float4* pairs;    // 4 per BVH node, filled for inner nodes N: the boxes of children L = N + 1 and
-                            // R = next(L): {L.min.xyz, L.max.x}, {L.max.yz, R.min.xy}, {R.min.z, R.max.xyz},
-                            // {L first triangle, R first triangle, R index, 0} (-1 inner, -2 empty leaf)
+                            // R = next(L): {L.min.xy, L.max.xy}, {R.min.xy, R.max.xy},
+                            // {L.min.z, L.max.z, R.min.z, R.max.z}, {L code, R code, R index, 0}; a code is the
+                            // child's index (inner), ~(first triangle) (leaf) or INT_MIN (empty leaf)
     int use_pairs;          // 1: every mesh BVH is a full binary tree, so pair records describe the walk;
-                            // 2: the same, and no leaf is empty (the compact pair walk's condition)
+                            // 2: the same, and no leaf is empty (the compact pair walk's condition);
+                            // 3: the same, children and triangles lie in their boxes and no tree is deeper
+                            // than DFPT_WALK_DEPTH (the packed pair walk's condition)
+    const int4* prim_walk;  // {shape type, shape offset, record index, first primitive of the run with this matrix}
     int pair_stack;         // entries of the compact pair walk's stack in use (1..8; 8 unless a test lowers it)
     const float4* shade_tris;  // per triangle (triangle offset / 12), the values surface() reads, copied from
                                // point3fs / point2fs / vector3fs: {a.xyz, b.x}, {b.yz, c.xy}, {c.z, uva.xy, uvb.x},
@@ -56,6 +60,7 @@ struct DevScene {
 };
 #define DFPT_CULL_CANDIDATES 16  // candidates a ray collects before falling back to the full loop
 #define DFPT_CULL_STACK 32
+#define DFPT_WALK_DEPTH 64  // levels below a mesh's root that the packed pair walk's stack holds
 
 // Renderer parameters and derived per-scene constants, in device memory (read through __ldg) so
 // captured CUDA graphs stay valid when they change.

@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(DevScene S0, const DevPar
             const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
             const Hit h = trace_v<ANY, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
             if (valid) __stcs(B.q_hit + i, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset));
-            warp_add_stats(P, B.stats, ANY ? 1 : 0, valid ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V != 6) warp_add_stats(P, B.stats, ANY ? 1 : 0, valid ? 1u : 0u, st.nodes, st.tris);
         }
     }
 }
@@ -1209,7 +1209,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow(DevScene S0, const DevPa
             const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
             const Hit h = trace_v<true, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
             if (valid && h.t >= INF - 0.0001f) unoccluded(i, o, __ldcs(B.s_c + i));
-            warp_add_stats(P, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V != 6) warp_add_stats(P, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
         }
     }
 }
@@ -1258,7 +1258,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_final(DevScene S0, const DevPar
             const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
             const Hit h = trace_v<true, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
             if (valid && !(h.t < INF)) escaped(o, d);
-            warp_add_stats(P0, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V != 6) warp_add_stats(P0, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
         }
     }
 }
@@ -1309,7 +1309,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
         {
             TraceStats st{0, 0};
             const Hit h = trace_v<false, V>(S, step, o.x, o.y, o.z, d.x, d.y, d.z, st);
-            warp_add_stats(P, B.stats, 0, step ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V != 6) warp_add_stats(P, B.stats, 0, step ? 1u : 0u, st.nodes, st.tris);
             bool emit_next = false, emit_shadow = false;
             float4 no = make_float4(0, 0, 0, 0), nd = make_float4(0, 0, 0, 0);
             float4 so = make_float4(0, 0, 0, 0), sd = make_float4(0, 0, 0, 0), sc = make_float4(0, 0, 0, 0);
@@ -1339,7 +1339,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
         if (__any_sync(0xFFFFFFFFu, fin)) {
             TraceStats st{0, 0};
             const Hit h = trace_v<true, V>(S, fin, o.x, o.y, o.z, d.x, d.y, d.z, st);
-            warp_add_stats(P, B.stats, 1, fin ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V != 6) warp_add_stats(P, B.stats, 1, fin ? 1u : 0u, st.nodes, st.tris);
             if (fin) {
                 if (!(h.t < INF)) {
                     const int path = __float_as_int(o.w);
@@ -1360,7 +1360,21 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
 // ---------------------------------------------------------------------------------------------
 // The per-pixel modes: ray caster, ambient occlusion, surface normals, ray tracer, ray marcher.
 
+// PACKED: the packed pair walk for every ray (nothing is counted), in a function of its own: k_simple
+// calls it from four places and needs few registers beside it (64 against 112, 8 blocks of 128 per SM
+// against 4: the 1080p ray-cast view of mesh_scene 1.80 -> 1.31 ms, ambient occlusion at 1003 x 601
+// 0.71 -> 0.50 ms with its readbacks).
+__device__ __noinline__ Hit trace_simple_packed(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz) {
+    return trace_pairs<false, 128>(S, ox, oy, oz, dx, dy, dz);
+}
+template <bool PACKED>
+__device__ __forceinline__ Hit trace_simple(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz, TraceStats& st) {
+    if constexpr (PACKED) return trace_simple_packed(S, ox, oy, oz, dx, dy, dz);
+    else return trace_s(S, ox, oy, oz, dx, dy, dz, st);
+}
+
 // doShaderPhongReflectionModel0 (GRK:1962-2039), with the reference's closest-hit shadow test.
+template <bool PACKED>
 __device__ int phong0(const DevScene& S, const DevParams& P, bool test, float px, float py, float pz, float nx, float ny, float nz,
                       float vx, float vy, float vz, float ar, float ag, float ab, TraceStats& st) {
     float r = 0.0f, g = 0.0f, b = 0.0f;
@@ -1371,7 +1385,7 @@ __device__ int phong0(const DevScene& S, const DevParams& P, bool test, float px
     const float lr = 1.0f / ll;
     const float lnx = lx * lr, lny = ly * lr, lnz = lz * lr;
     float t = INF;
-    if (test) t = trace_s(S, px, py, pz, lnx, lny, lnz, st).t;
+    if (test) t = trace_simple<PACKED>(S, px, py, pz, lnx, lny, lnz, st).t;
     if (t >= INF || t > l2) {
         const float ldn = lnx * nx + lny * ny + lnz * nz;
         r += ar * 0.5f * jmax(ldn, 0.0f) * 1.0f;
@@ -1404,7 +1418,8 @@ __device__ float height_rm(const DevParams& P, float x, float z) {
     return fractal2(P.g_amplitude, P.g_frequency, P.g_gain, P.g_lacunarity, P.g_octaves, x, z);
 }
 
-__global__ void __launch_bounds__(128) k_simple(DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
+template <bool PACKED>
+__global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
     const DevParams& P = *Pp;
     const int n = B.n_pixels;
     const uint32_t pass = (uint32_t)*B.pass_index;
@@ -1439,7 +1454,7 @@ __global__ void __launch_bounds__(128) k_simple(DevScene S, const DevParams* __r
                             const float nr = 1.0f / sqrtf(nx * nx + ny * ny + nz * nz);
                             const float noise = fbm3(8.0f, 0.5f, 0.0f, 1.0f, 16, px, py, pz);
                             const float al = saturate_j(noise * 1.0f + 0.1f, 0.0f, 1.0f);
-                            const int c = phong0(S, P, false, px, py, pz, nx * nr, ny * nr, nz * nr, -dx, -dy, -dz, al, al, al, st);
+                            const int c = phong0<PACKED>(S, P, false, px, py, pz, nx * nr, ny * nr, nz * nr, -dx, -dy, -dz, al, al, al, st);
                             cr_ = cr(c); cg_ = cg(c); cb_ = cb(c);
                             t = max_t;
                         }
@@ -1448,7 +1463,7 @@ __global__ void __launch_bounds__(128) k_simple(DevScene S, const DevParams* __r
                 } else {
                     const int depth_max = mode == DFPT_RENDERER_RAY_TRACER ? 5 : 1;
                     for (int depth = 0; depth < depth_max; ++depth) {
-                        const Hit h = trace_s(S, ox, oy, oz, dx, dy, dz, st);
+                        const Hit h = trace_simple<PACKED>(S, ox, oy, oz, dx, dy, dz, st);
                         segs++;
                         if (depth == 0) B.primitive_offsets[i] = h.prim >= 0 ? h.prim * 3 : -1;
                         if (h.t == INF || h.prim == -1) {
@@ -1487,7 +1502,7 @@ __global__ void __launch_bounds__(128) k_simple(DevScene S, const DevParams* __r
                             const float e1z = e0x * u2z + e0y * v0z + e0z * w1z;
                             const float er = rsqrt_j(e1x * e1x + e1y * e1y + e1z * e1z);
                             const float aox = s.px + w1x * 0.01f, aoy = s.py + w1y * 0.01f, aoz = s.pz + w1z * 0.01f;
-                            const float t = trace_s(S, aox, aoy, aoz, e1x * er, e1y * er, e1z * er, st).t;
+                            const float t = trace_simple<PACKED>(S, aox, aoy, aoz, e1x * er, e1y * er, e1z * er, st).t;
                             segs++;
                             const bool hit = t < P.ao_max_distance;
                             const float v = hit ? 1.0f : 0.0f;  // bright 1, dark 0
@@ -1504,7 +1519,7 @@ __global__ void __launch_bounds__(128) k_simple(DevScene S, const DevParams* __r
                         } else {
                             ar = cr(albedo); ag = cg(albedo); ab = cb(albedo);
                         }
-                        const int c = phong0(S, P, true, s.px, s.py, s.pz, wx, wy, wz, -dx, -dy, -dz, ar, ag, ab, st);
+                        const int c = phong0<PACKED>(S, P, true, s.px, s.py, s.pz, wx, wy, wz, -dx, -dy, -dz, ar, ag, ab, st);
                         segs++;
                         if (mode == DFPT_RENDERER_RAY_CASTER) {
                             cr_ = cr(c); cg_ = cg(c); cb_ = cb(c);
@@ -1523,7 +1538,7 @@ __global__ void __launch_bounds__(128) k_simple(DevScene S, const DevParams* __r
             B.radiance[PSI(i)] = make_float4(cr_, cg_, cb_, 0.0f);
             B.rng[i] = rng.state;
         }
-        warp_add_stats(P, B.stats, 0, segs, st.nodes, st.tris);
+        if constexpr (!PACKED) warp_add_stats(P, B.stats, 0, segs, st.nodes, st.tris);
     }
 }
 
@@ -2000,24 +2015,55 @@ __global__ void k_init_tables(const int* perm256, const float* grad36) {
 #define BATCH_SCENE(c) DevScene{}
 #endif
 
+// A grid of every block of `kernel` that the current device holds at once.
+template <class Kernel>
+static int resident_grid(Kernel kernel, int block) {
+    int dev = 0, sms = 0, b = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, block, 0);
+    return (sms > 0 ? sms : 1) * (b > 0 ? b : 1);
+}
+
 template <int V, int BLOCK, int MINB>
 struct TraceCfg {
     static void carveout(int percent) {
 #ifndef DFPT_ONE_SCENE
         cudaFuncSetAttribute(k_trace<false, false, V, BLOCK, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+        if constexpr (V == 5) cudaFuncSetAttribute(k_trace<false, false, 6, BLOCK, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
 #endif
 #ifdef DFPT_EXTENDED_KERNELS
         cudaFuncSetAttribute(k_trace<true, false, (V == 2 ? 1 : V), BLOCK, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+        if constexpr (V == 5) cudaFuncSetAttribute(k_trace<true, false, 6, BLOCK, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
 #endif
     }
 #ifndef DFPT_ONE_SCENE
+    // Configurations of the compact pair walk (V 5) launch the packed pair walk (6) where it may run.
     static void closest(const LaunchCtx& c, int bounce) {
+        if constexpr (V == 5) {
+            if (c.packed) {
+                k_trace<false, false, 6, BLOCK, MINB><<<resident_grid(k_trace<false, false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                return;
+            }
+        }
         k_trace<false, false, V, BLOCK, MINB><<<c.grid_trace, BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
     }
     static void shadow(const LaunchCtx& c, int bounce) {
+        if constexpr (V == 5) {
+            if (c.packed) {
+                k_shadow<false, 6, BLOCK, MINB><<<resident_grid(k_shadow<false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                return;
+            }
+        }
         k_shadow<false, V, BLOCK, MINB><<<c.grid_trace, BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
     }
     static void final_(const LaunchCtx& c, int bounce) {
+        if constexpr (V == 5) {
+            if (c.packed) {
+                k_final<false, 6, BLOCK, MINB><<<resident_grid(k_final<false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                return;
+            }
+        }
         k_final<false, V, BLOCK, MINB><<<c.grid_trace, BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
     }
     static int grid(int sms) {
@@ -2027,22 +2073,19 @@ struct TraceCfg {
     }
     // The tail kernel: traversal and shading in one kernel, compiled for 2 resident blocks of 256,
     // and with the compact pair walk of the fast set also for 3 or 4 (c.tail_blocks: fewer
-    // registers, more warps to hide the walk's load latency); its grid (SMs x resident blocks) is
-    // found once per process. Its walk is the configuration's when that is the threaded walk (0)
+    // registers, more warps to hide the walk's load latency). Its walk is the configuration's when that is the threaded walk (0)
     // or the compact pair walk (5), else the prefetching walk (1), so that three walks serve every
     // configuration (the other walks lost to these in whole launches).
     static constexpr int TVV = (V == 0 || V == 5) ? V : 1;
     template <int TB>
     static void tail_t(const LaunchCtx& c, int b0, int nb) {
-        static int grid_tail = 0;
-        if (grid_tail == 0) {
-            int dev = 0, sms = 0, b = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_tail<TVV, 256, TB>, 256, 0);
-            grid_tail = (sms > 0 ? sms : 1) * (b > 0 ? b : 1);
+        if constexpr (TVV == 5) {
+            if (c.packed) {
+                k_tail<6, 256, TB><<<resident_grid(k_tail<6, 256, TB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
+                return;
+            }
         }
-        k_tail<TVV, 256, TB><<<grid_tail, 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
+        k_tail<TVV, 256, TB><<<resident_grid(k_tail<TVV, 256, TB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
     }
     static void tail(const LaunchCtx& c, int b0, int nb) {
 #ifdef DFPT_EXTENDED_KERNELS
@@ -2058,12 +2101,30 @@ struct TraceCfg {
     // Batch traversal: per-lane walks only (a warp may hold rays of several scenes).
     static constexpr int BV = V == 2 ? 1 : V;
     static void b_closest(const LaunchCtx& c, int bounce) {
+        if constexpr (BV == 5) {
+            if (c.packed) {
+                k_trace<true, false, 6, BLOCK, MINB><<<resident_grid(k_trace<true, false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                return;
+            }
+        }
         k_trace<true, false, BV, BLOCK, MINB><<<c.grid_trace, BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
     }
     static void b_shadow(const LaunchCtx& c, int bounce) {
+        if constexpr (BV == 5) {
+            if (c.packed) {
+                k_shadow<true, 6, BLOCK, MINB><<<resident_grid(k_shadow<true, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                return;
+            }
+        }
         k_shadow<true, BV, BLOCK, MINB><<<c.grid_trace, BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
     }
     static void b_final(const LaunchCtx& c, int bounce) {
+        if constexpr (BV == 5) {
+            if (c.packed) {
+                k_final<true, 6, BLOCK, MINB><<<resident_grid(k_final<true, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                return;
+            }
+        }
         k_final<true, BV, BLOCK, MINB><<<c.grid_trace, BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
     }
 #ifdef DFPT_ONE_SCENE
@@ -2199,7 +2260,10 @@ static void launch_diff_reduce(const LaunchCtx& c, const double* rows, int n_row
 }
 #endif
 #ifndef DFPT_ONE_SCENE
-static void launch_simple(const LaunchCtx& c) { k_simple<<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass); }
+static void launch_simple(const LaunchCtx& c) {
+    if (c.packed) k_simple<true><<<resident_grid(k_simple<true>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    else k_simple<false><<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+}
 static void launch_wireframe(const LaunchCtx& c) { k_wireframe<<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass); }
 static void launch_film(const LaunchCtx& c) { k_film<<<c.grid, 256, 0, c.stream>>>(c.params, *c.pass); }
 static void launch_end_pass(const LaunchCtx& c) { k_end_pass<<<1, 32, 0, c.stream>>>(*c.pass); }
@@ -2234,7 +2298,7 @@ static void occupancy(int sms, int& grid, int& grid_trace, int& grid_simple) {
     b3 = b1;
 #else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_shade<false>, 256, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, k_simple, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, k_simple<false>, 128, 0);
 #endif
     grid = sms * (b1 > 0 ? b1 : 1);
     grid_trace = trace_grid(0, sms);

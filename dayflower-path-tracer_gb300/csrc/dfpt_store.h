@@ -71,7 +71,8 @@ struct SceneStore {
     Derived derived;  // emptied once uploaded
     DevBuf<float> point2fs, point3fs, vector3fs, spheres, terrains, textures, surfaces, o2w, w2o, camera;
     DevBuf<int> planes, triangles, primitives;
-    DevBuf<int4> prim_info;
+    DevBuf<int4> prim_info;  // DevScene::prim_info, then DevScene::prim_walk
+    std::vector<int4> prim_info_host;
     DevBuf<float4> trav;  // BVH nodes then triangles, one allocation (one L2 persistence window)
     DevBuf<float4> pairs;  // per node: the children's boxes (pair records, see DevScene::pairs)
     DevBuf<float4> shade_tris;  // per triangle: the vertex values shading reads (see DevScene::shade_tris)
@@ -93,6 +94,8 @@ int scene_upload(SceneStore& st, cudaStream_t s);
 // Selects the primitive culling mode in st.scene (0 none, 1 box test, 2 BVH candidates; 0 when
 // the scene has too few bounded primitives).
 void scene_set_culling(SceneStore& st, int mode);
+// Brings prim_walk (each primitive's run of equal world-to-object matrices) up to date after the matrices changed.
+int scene_update_walk(SceneStore& st, cudaStream_t s);
 // Rebuilds the culling structure after the world-to-object matrices changed.
 int scene_rebuild_culling(SceneStore& st, cudaStream_t s);
 int culling_upload(SceneStore& st, const Derived& d, cudaStream_t s);
