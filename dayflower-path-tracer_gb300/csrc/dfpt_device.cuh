@@ -111,6 +111,12 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint2 k) {
     return c;
 }
 
+// The generator's block as a function of its own: a path draws at up to ten places, and the ten
+// rounds inlined at each made the shading kernels miss the instruction cache.
+__device__ __noinline__ uint4 philox_block(uint32_t pass, uint32_t bid, uint32_t seed_hi, uint32_t pixel, uint32_t seed_lo) {
+    return philox4x32_10(make_uint4(pass, bid, seed_hi, 0x44465054u), make_uint2(pixel, seed_lo));
+}
+
 struct Rng {
     uint64_t state;  // LCG: 48-bit state; counter: draws made this pass
     uint32_t pixel, pass, seed_lo, seed_hi;
@@ -127,7 +133,7 @@ struct Rng {
         state = (uint64_t)(i + 1u);
         const uint32_t bid = i >> 2;
         if (bid != block_id) {
-            block = philox4x32_10(make_uint4(pass, bid, seed_hi, 0x44465054u), make_uint2(pixel, seed_lo));
+            block = philox_block(pass, bid, seed_hi, pixel, seed_lo);
             block_id = bid;
         }
         const uint32_t lane = i & 3u;

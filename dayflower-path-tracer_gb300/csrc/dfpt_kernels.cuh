@@ -26,9 +26,10 @@ __device__ __forceinline__ float3 v3(const DevScene& S, int off) {
     return make_float3(__ldg(S.vector3fs + off), __ldg(S.vector3fs + off + 1), __ldg(S.vector3fs + off + 2));
 }
 __device__ __forceinline__ float texf(const DevScene& S, int off) { return __ldg(S.textures + off); }
+__device__ __forceinline__ float texf(const float* textures, int off) { return __ldg(textures + off); }
 
 // Image texture lookup without filtering (GRK:1894-1929).
-__device__ int image_texture_simple(const DevScene& S, int to, float u, float v) {
+__device__ int image_texture_simple(const float* S, int to, float u, float v) {
     const float width = texf(S, to + 4), height = texf(S, to + 5);
     const float su = texf(S, to + 6), sv = texf(S, to + 7);
     const float ca = texf(S, to + 2), sa = texf(S, to + 3);
@@ -40,6 +41,72 @@ __device__ int image_texture_simple(const DevScene& S, int to, float u, float v)
     const int w = f2i(width), res = f2i(width * height);
     const int index = y * w + x;
     return index >= 0 && index < res ? f2i(texf(S, to + 8 + index)) : 0;
+}
+
+__device__ __noinline__ Surf terrain_surface(float oxo, float oyo, float ozo, float dxo, float dyo, float dzo, float t) {
+    Surf s;
+    s.tx = s.ty = s.tz = 0.0f;
+    const float sr = 1.0f / 10.0f;
+    s.px = oxo * sr + dxo * t; s.py = oyo * sr + dyo * t; s.pz = ozo * sr + dzo * t;
+    const float e = 0.02f;
+    const float nx = (sin_j(s.px - e) * sin_j(s.pz)) - (sin_j(s.px + e) * sin_j(s.pz));
+    const float ny = 2.0f * e;
+    const float nz = (sin_j(s.px) * sin_j(s.pz - e)) - (sin_j(s.px) * sin_j(s.pz + e));
+    const float r = rsqrt_j(nx * nx + ny * ny + nz * nz);
+    s.nx = nx * r; s.ny = ny * r; s.nz = nz * r;
+    s.u = s.px; s.v = s.pz;
+    return s;
+}
+
+// Normal mapping via an image texture (GRK:2714-2846) and via noise (GRK:2658-2712).
+__device__ __noinline__ float3 normal_map_image(const float* S, int shape_type, int nto, const Surf s) {
+    const int rgb = image_texture_simple(S, nto, s.u, s.v);
+    const float r = ((((rgb >> 16) & 0xFF) * COLOR_RECIPROCAL) - 0.5f) * 2.0f;
+    const float g = ((((rgb >> 8) & 0xFF) * COLOR_RECIPROCAL) - 0.5f) * 2.0f;
+    const float bb = ((((rgb >> 0) & 0xFF) * COLOR_RECIPROCAL) - 0.0f) * 2.0f;
+    const float wx = s.nx, wy = s.ny, wz = s.nz;
+    float sx, sy, sz;
+    if (shape_type == DFPT_SHAPE_SPHERE) {
+        const float v0x = -2.0f * PI_F * wy, v0y = 2.0f * PI_F * wx, v0z = 0.0f;
+        const float u0x = v0y * wz - v0z * wy, u0y = v0z * wx - v0x * wz, u0z = v0x * wy - v0y * wx;
+        const float ur = rsqrt_j(u0x * u0x + u0y * u0y + u0z * u0z);
+        const float u1x = u0x * ur, u1y = u0y * ur, u1z = u0z * ur;
+        const float v1x = wy * u1z - wz * u1y, v1y = wz * u1x - wx * u1z, v1z = wx * u1y - wy * u1x;
+        const float vr = rsqrt_j(v1x * v1x + v1y * v1y + v1z * v1z);
+        const float v2x = v1x * vr, v2y = v1y * vr, v2z = v1z * vr;
+        sx = r * u1x + g * v2x + bb * wx; sy = r * u1y + g * v2y + bb * wy; sz = r * u1z + g * v2z + bb * wz;
+    } else if (shape_type == DFPT_SHAPE_TRIANGLE) {
+        const float ux = s.tx, uy = s.ty, uz = s.tz;
+        const float v0x = wy * uz - wz * uy, v0y = wz * ux - wx * uz, v0z = wx * uy - wy * ux;
+        const float vr = rsqrt_j(v0x * v0x + v0y * v0y + v0z * v0z);
+        const float v1x = v0x * vr, v1y = v0y * vr, v1z = v0z * vr;
+        sx = r * ux + g * v1x + bb * wx; sy = r * uy + g * v1y + bb * wy; sz = r * uz + g * v1z + bb * wz;
+    } else {
+        const float awx = fabsf(wx), awy = fabsf(wy), awz = fabsf(wz);
+        const bool isWX = awx < awy && awx < awz;
+        const bool isWY = awy < awz;
+        const float v0x = isWX ? 0.0f : isWY ? wz : wy;
+        const float v0y = isWX ? wz : isWY ? 0.0f : -wx;
+        const float v0z = isWX ? -wy : isWY ? -wx : 0.0f;
+        const float vr = rsqrt_j(v0x * v0x + v0y * v0y + v0z * v0z);
+        const float v1x = v0x * vr, v1y = v0y * vr, v1z = v0z * vr;
+        const float u0x = v1y * wz - v1z * wy, u0y = v1z * wx - v1x * wz, u0z = v1x * wy - v1y * wx;
+        const float ur = rsqrt_j(u0x * u0x + u0y * u0y + u0z * u0z);
+        const float u1x = u0x * ur, u1y = u0y * ur, u1z = u0z * ur;
+        sx = r * u1x + g * v1x + bb * wx; sy = r * u1y + g * v1y + bb * wy; sz = r * u1z + g * v1z + bb * wz;
+    }
+    const float sr = rsqrt_j(sx * sx + sy * sy + sz * sz);
+    return make_float3(sx * sr, sy * sr, sz * sr);
+}
+__device__ __noinline__ float3 normal_map_noise(float amount, float scale, const Surf s) {
+    const float sr = 1.0f / scale;
+    const float x1 = s.px * sr, y1 = s.py * sr, z1 = s.pz * sr;
+    const float nx = fbm3(scale, 0.5f, -0.26f, 0.26f, 16, x1, y1, z1);
+    const float ny = fbm3(scale, 0.5f, -0.26f, 0.26f, 16, y1, z1, x1);
+    const float nz = fbm3(scale, 0.5f, -0.26f, 0.26f, 16, z1, x1, y1);
+    const float qx = s.nx + nx * amount, qy = s.ny + ny * amount, qz = s.nz + nz * amount;
+    const float qr = rsqrt_j(qx * qx + qy * qy + qz * qz);
+    return make_float3(qx * qr, qy * qr, qz * qr);
 }
 
 // Object-space surface properties of the hit, the transform to world space and normal mapping
@@ -91,15 +158,7 @@ __device__ Surf surface(const DevScene& S, const DevParams& P, float ox, float o
         s.u = 0.5f + atan2_j(-s.nz, -s.nx) * INV_TWO_PI;
         s.v = 0.5f - asin_j(-s.ny) * INV_PI;
     } else if (h.shape_type == DFPT_SHAPE_TERRAIN) {
-        const float sr = 1.0f / 10.0f;
-        s.px = oxo * sr + dxo * t; s.py = oyo * sr + dyo * t; s.pz = ozo * sr + dzo * t;
-        const float e = 0.02f;
-        const float nx = (sin_j(s.px - e) * sin_j(s.pz)) - (sin_j(s.px + e) * sin_j(s.pz));
-        const float ny = 2.0f * e;
-        const float nz = (sin_j(s.px) * sin_j(s.pz - e)) - (sin_j(s.px) * sin_j(s.pz + e));
-        const float r = rsqrt_j(nx * nx + ny * ny + nz * nz);
-        s.nx = nx * r; s.ny = ny * r; s.nz = nz * r;
-        s.u = s.px; s.v = s.pz;
+        s = terrain_surface(oxo, oyo, ozo, dxo, dyo, dzo, t);
     } else {  // Triangle
         // The vertex values come from the triangle's shading record (one contiguous 144-byte
         // record, the same floats) when the scene has them, else through the reference's indices.
@@ -183,58 +242,15 @@ __device__ Surf surface(const DevScene& S, const DevParams& P, float ox, float o
     const int4 info = __ldg(S.prim_info + h.prim);
     const int so = info.z;
     if (P.normal_mapping == 1) {
-        // Normal mapping via image texture (GRK:2714-2846).
         const int nto = f2i(__ldg(S.surfaces + so + 3));
         if (f2i(texf(S, nto)) == DFPT_TEXTURE_IMAGE) {
-            const int rgb = image_texture_simple(S, nto, s.u, s.v);
-            const float r = ((((rgb >> 16) & 0xFF) * COLOR_RECIPROCAL) - 0.5f) * 2.0f;
-            const float g = ((((rgb >> 8) & 0xFF) * COLOR_RECIPROCAL) - 0.5f) * 2.0f;
-            const float bb = ((((rgb >> 0) & 0xFF) * COLOR_RECIPROCAL) - 0.0f) * 2.0f;
-            const float wx = s.nx, wy = s.ny, wz = s.nz;
-            float sx, sy, sz;
-            if (info.x == DFPT_SHAPE_SPHERE) {
-                const float v0x = -2.0f * PI_F * wy, v0y = 2.0f * PI_F * wx, v0z = 0.0f;
-                const float u0x = v0y * wz - v0z * wy, u0y = v0z * wx - v0x * wz, u0z = v0x * wy - v0y * wx;
-                const float ur = rsqrt_j(u0x * u0x + u0y * u0y + u0z * u0z);
-                const float u1x = u0x * ur, u1y = u0y * ur, u1z = u0z * ur;
-                const float v1x = wy * u1z - wz * u1y, v1y = wz * u1x - wx * u1z, v1z = wx * u1y - wy * u1x;
-                const float vr = rsqrt_j(v1x * v1x + v1y * v1y + v1z * v1z);
-                const float v2x = v1x * vr, v2y = v1y * vr, v2z = v1z * vr;
-                sx = r * u1x + g * v2x + bb * wx; sy = r * u1y + g * v2y + bb * wy; sz = r * u1z + g * v2z + bb * wz;
-            } else if (info.x == DFPT_SHAPE_TRIANGLE) {
-                const float ux = s.tx, uy = s.ty, uz = s.tz;
-                const float v0x = wy * uz - wz * uy, v0y = wz * ux - wx * uz, v0z = wx * uy - wy * ux;
-                const float vr = rsqrt_j(v0x * v0x + v0y * v0y + v0z * v0z);
-                const float v1x = v0x * vr, v1y = v0y * vr, v1z = v0z * vr;
-                sx = r * ux + g * v1x + bb * wx; sy = r * uy + g * v1y + bb * wy; sz = r * uz + g * v1z + bb * wz;
-            } else {
-                const float awx = fabsf(wx), awy = fabsf(wy), awz = fabsf(wz);
-                const bool isWX = awx < awy && awx < awz;
-                const bool isWY = awy < awz;
-                const float v0x = isWX ? 0.0f : isWY ? wz : wy;
-                const float v0y = isWX ? wz : isWY ? 0.0f : -wx;
-                const float v0z = isWX ? -wy : isWY ? -wx : 0.0f;
-                const float vr = rsqrt_j(v0x * v0x + v0y * v0y + v0z * v0z);
-                const float v1x = v0x * vr, v1y = v0y * vr, v1z = v0z * vr;
-                const float u0x = v1y * wz - v1z * wy, u0y = v1z * wx - v1x * wz, u0z = v1x * wy - v1y * wx;
-                const float ur = rsqrt_j(u0x * u0x + u0y * u0y + u0z * u0z);
-                const float u1x = u0x * ur, u1y = u0y * ur, u1z = u0z * ur;
-                sx = r * u1x + g * v1x + bb * wx; sy = r * u1y + g * v1y + bb * wy; sz = r * u1z + g * v1z + bb * wz;
-            }
-            const float sr = rsqrt_j(sx * sx + sy * sy + sz * sz);
-            s.nx = sx * sr; s.ny = sy * sr; s.nz = sz * sr;
+            const float3 n = normal_map_image(S.textures, info.x, nto, s);
+            s.nx = n.x; s.ny = n.y; s.nz = n.z;
         }
-        // Normal mapping via noise (GRK:2658-2712).
         const float amount = __ldg(S.surfaces + so + 4), scale = __ldg(S.surfaces + so + 5);
         if (amount > 0.0f && scale > 0.0f) {
-            const float sr = 1.0f / scale;
-            const float x1 = s.px * sr, y1 = s.py * sr, z1 = s.pz * sr;
-            const float nx = fbm3(scale, 0.5f, -0.26f, 0.26f, 16, x1, y1, z1);
-            const float ny = fbm3(scale, 0.5f, -0.26f, 0.26f, 16, y1, z1, x1);
-            const float nz = fbm3(scale, 0.5f, -0.26f, 0.26f, 16, z1, x1, y1);
-            const float qx = s.nx + nx * amount, qy = s.ny + ny * amount, qz = s.nz + nz * amount;
-            const float qr = rsqrt_j(qx * qx + qy * qy + qz * qz);
-            s.nx = qx * qr; s.ny = qy * qr; s.nz = qz * qr;
+            const float3 n = normal_map_noise(amount, scale, s);
+            s.nx = n.x; s.ny = n.y; s.nz = n.z;
         }
     }
     return s;
@@ -253,7 +269,7 @@ __device__ __forceinline__ float cr(int rgb) { return ((rgb >> 16) & 0xFF) * COL
 __device__ __forceinline__ float cg(int rgb) { return ((rgb >> 8) & 0xFF) * COLOR_RECIPROCAL; }
 __device__ __forceinline__ float cb(int rgb) { return (rgb & 0xFF) * COLOR_RECIPROCAL; }
 
-__device__ int texture_leaf(const DevScene& S, int to, const Surf& s) {
+__device__ __noinline__ int texture_leaf(const float* S, int to, const Surf s) {
     const int type = f2i(texf(S, to));
     if (type == DFPT_TEXTURE_BULLSEYE) {
         const int ca = f2i(texf(S, to + 2)), cbb = f2i(texf(S, to + 3));
@@ -307,7 +323,7 @@ __device__ int texture_leaf(const DevScene& S, int to, const Surf& s) {
     return 0;
 }
 
-__device__ int texture_color(const DevScene& S, int to, const Surf& s) {
+__device__ __noinline__ int texture_blend_or_leaf(const float* S, int to, const Surf s) {
     if (f2i(texf(S, to)) == DFPT_TEXTURE_BLEND) {
         const int ta = f2i(texf(S, to + 2)), tb = f2i(texf(S, to + 3));
         const float f = texf(S, to + 4);
@@ -315,6 +331,14 @@ __device__ int texture_color(const DevScene& S, int to, const Surf& s) {
         return pack8((1.0f - f) * cr(a) + f * cr(b), (1.0f - f) * cg(a) + f * cg(b), (1.0f - f) * cb(a) + f * cb(b));
     }
     return texture_leaf(S, to, s);
+}
+
+// The color of a surface's texture. Constant textures, by far the most common, are read in place; the
+// other kinds (fBm noise, images, blends) are functions of their own: inlined at their six places they
+// made k_shade 187 KB of code.
+__device__ __forceinline__ int texture_color(const DevScene& S, int to, const Surf& s) {
+    if (f2i(texf(S, to)) == DFPT_TEXTURE_CONSTANT) return f2i(texf(S, to + 2));
+    return texture_blend_or_leaf(S.textures, to, s);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -361,6 +385,9 @@ __device__ float3 sky_color(const DevParams& P, float dx, float dy, float dz) {
     return c;
 }
 
+// {cos, sin} of a sampled azimuth, one copy for all the places that draw one.
+__device__ __noinline__ float2 azimuth(float phi) { return make_float2(cos_j(phi), sin_j(phi)); }
+
 // Sun sample of doCalculateColorForSun (GRK:2238-2347): a direction in the 500-radius cone
 // around the sun direction; returns false when the sample faces away from the sun or surface.
 __device__ bool sun_sample(const DevParams& P, float px, float py, float pz, float nx, float ny, float nz, float u, float v,
@@ -372,8 +399,8 @@ __device__ bool sun_sample(const DevParams& P, float px, float py, float pz, flo
     const float cos_max = sqrtf(jmax(0.0f, 1.0f - sin2));
     const float cos_t = u * (cos_max - 1.0f) + 1.0f;
     const float sin_t = sqrtf(jmax(0.0f, 1.0f - cos_t * cos_t));
-    const float phi = TWO_PI * v;
-    const float x = cos_j(phi) * sin_t, y = sin_j(phi) * sin_t, z = cos_t;
+    const float2 cs = azimuth(TWO_PI * v);
+    const float x = cs.x * sin_t, y = cs.y * sin_t, z = cos_t;
     const float wx = P.sun_dir_world[0], wy = P.sun_dir_world[1], wz = P.sun_dir_world[2];
     const float ax = fabsf(wx), ay = fabsf(wy), az = fabsf(wz);
     const float vx = ax < ay && ax < az ? 0.0f : ay < az ? wz : wy;
@@ -394,9 +421,9 @@ __device__ bool sun_sample(const DevParams& P, float px, float py, float pz, flo
 
 // Cosine-weighted hemisphere direction around w (GRK:3466-3500).
 __device__ __forceinline__ void cosine_dir(float wx, float wy, float wz, float u, float v, float& ox, float& oy, float& oz) {
-    const float phi = TWO_PI * u;
+    const float2 cs = azimuth(TWO_PI * u);
     const float ct = sqrtf(v), st = sqrtf(1.0f - v);
-    const float x = cos_j(phi) * st, y = sin_j(phi) * st, z = ct;
+    const float x = cs.x * st, y = cs.y * st, z = ct;
     const bool isY = fabsf(wx) > 0.1f;
     const float ux = (isY ? 1.0f : 0.0f) * wz;
     const float uy = -((isY ? 0.0f : 1.0f) * wz);
@@ -811,6 +838,7 @@ __device__ __forceinline__ Scatter scatter(const Surf& s, int material, float wx
     out.phong_ct = 0.0f;
     float ox = o.x, oy = o.y, oz = o.z, dx = d.x, dy = d.y, dz = d.z;
     const float rx = dx - s.nx * dp2, ry = dy - s.ny * dp2, rz = dz - s.nz * dp2;
+    bool diffuse = false;  // a cosine-distributed direction, sampled below for both materials that have one
     if (material == DFPT_MATERIAL_CLEAR_COAT) {
         const float a = 1.5f - 1.0f, b = 1.5f + 1.0f, c = 1.0f / 1.5f;
         const float e = (a * a) / (b * b);
@@ -832,26 +860,18 @@ __device__ __forceinline__ Scatter scatter(const Surf& s, int material, float wx
                 ox = s.px + wx * 0.02f; oy = s.py + wy * 0.02f; oz = s.pz + wz * 0.02f;
                 dx = rx; dy = ry; dz = rz;
             } else {
-                const float u = rng.next(), v = rng.next();
-                cosine_dir(wx, wy, wz, u, v, dx, dy, dz);
-                ox = s.px + wx * 0.01f; oy = s.py + wy * 0.01f; oz = s.pz + wz * 0.01f;
-                T.x *= ar; T.y *= ag; T.z *= ab;
-                out.albedo = true;
+                diffuse = true;
             }
         }
     } else if (material == DFPT_MATERIAL_LAMBERTIAN) {
-        const float u = rng.next(), v = rng.next();
-        cosine_dir(wx, wy, wz, u, v, dx, dy, dz);
-        ox = s.px + wx * 0.01f; oy = s.py + wy * 0.01f; oz = s.pz + wz * 0.01f;
-        T.x *= ar; T.y *= ag; T.z *= ab;
-        out.albedo = true;
+        diffuse = true;
     } else if (material == DFPT_MATERIAL_PHONG) {
         const float u = rng.next(), v = rng.next();
-        const float phi = TWO_PI * u;
+        const float2 cs = azimuth(TWO_PI * u);
         const float ct = pow_j(1.0f - v, 1.0f / (exponent + 1.0f));
         out.phong_ct = ct;
         const float st = sqrtf(jmax(0.0f, 1.0f - ct * ct));
-        const float x = cos_j(phi) * st, y = sin_j(phi) * st, z = ct;
+        const float x = cs.x * st, y = cs.y * st, z = ct;
         const float rwr = rsqrt_j(rx * rx + ry * ry + rz * rz);
         const float rnx = rx * rwr, rny = ry * rwr, rnz = rz * rwr;
         const bool isY = fabsf(rnx) > 0.1f;
@@ -902,6 +922,13 @@ __device__ __forceinline__ Scatter scatter(const Surf& s, int material, float wx
     } else if (material == DFPT_MATERIAL_REFLECTION) {
         ox = s.px + s.nx * 0.000001f; oy = s.py + s.ny * 0.000001f; oz = s.pz + s.nz * 0.000001f;
         dx = rx; dy = ry; dz = rz;
+        T.x *= ar; T.y *= ag; T.z *= ab;
+        out.albedo = true;
+    }
+    if (diffuse) {
+        const float u = rng.next(), v = rng.next();
+        cosine_dir(wx, wy, wz, u, v, dx, dy, dz);
+        ox = s.px + wx * 0.01f; oy = s.py + wy * 0.01f; oz = s.pz + wz * 0.01f;
         T.x *= ar; T.y *= ag; T.z *= ab;
         out.albedo = true;
     }
@@ -1419,7 +1446,7 @@ __device__ float height_rm(const DevParams& P, float x, float z) {
 }
 
 template <bool PACKED>
-__global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
+__global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(const __grid_constant__ DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
     const DevParams& P = *Pp;
     const int n = B.n_pixels;
     const uint32_t pass = (uint32_t)*B.pass_index;
