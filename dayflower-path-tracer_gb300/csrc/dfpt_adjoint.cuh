@@ -199,7 +199,7 @@ __device__ void sun_rim_tan(const DevScene& S, const DevParams& P, uint32_t pixe
     float g_rim = 0.0f;
     if (dot0 > 0.0f && dot1 > 0.0f && c != 0.0f) {
         TraceStats st{0, 0};
-        const Hit h = trace_v<true, 1>(S, true, px, py, pz, rx, ry, rz, st);
+        const Hit h = S.flat ? trace_flat<true>(S, px, py, pz, rx, ry, rz) : trace_v<true, 1>(S, true, px, py, pz, rx, ry, rz, st);
         if (h.t >= INF - 0.0001f) g_rim = c * dot1;
     }
     const float k = (g_rim - g_forward) / one_m_cos;
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(256) k_final_adj(DevScene S, const DevParams* 
             o = B.q_o[qi][i];
             d = B.q_d[qi][i];
         }
-        const Hit h = trace_v<true, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
+        const Hit h = S.flat && valid ? trace_flat<true>(S, o.x, o.y, o.z, d.x, d.y, d.z) : trace_v<true, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
         if (valid && !(h.t < INF)) {
             const int path = __float_as_int(o.w);
             const float4 T = B.throughput[PSI(path)];

@@ -714,11 +714,12 @@ void mark(dfpt_handle* h, int kind) {
     h->events_used++;
 }
 
-// Whether the launches take the packed pair walk: it counts nothing and has no settable stack depth.
-void refresh_packed(dfpt_handle* h) {
-    const bool packed = h->sc.scene.use_pairs == 3 && !h->counting && h->sc.scene.pair_stack == 8;
-    if (packed == h->ctx.packed) return;
-    h->ctx.packed = packed;
+// The walk of the launches (LaunchCtx::walk): the counting walks while counting or with a set stack depth.
+void refresh_walk(dfpt_handle* h) {
+    const DevScene& S = h->sc.scene;
+    const int walk = h->counting ? 0 : S.flat ? 7 : S.use_pairs == 3 && S.pair_stack == 8 ? 6 : 0;
+    if (walk == h->ctx.walk) return;
+    h->ctx.walk = walk;
     h->graph_valid = false;
     h->wide_graph_valid = false;
 }
@@ -1409,6 +1410,8 @@ int scene_upload(SceneStore& st, cudaStream_t s) {
     S.textures = st.textures.p; S.surfaces = st.surfaces.p; S.primitives = st.primitives.p;
     S.o2w = st.o2w.p; S.w2o = st.w2o.p; S.camera = st.camera.p;
     S.prim_info = st.prim_info.p;
+    S.flat = 1;
+    for (const int4& info : d.prim_info) S.flat = info.x == DFPT_SHAPE_TRIANGLE_MESH ? 0 : S.flat;
     S.prim_walk = st.prim_info.p + d.prim_info.size();
     S.nodes = st.trav.p; S.tris = st.trav.p + st.trav_nodes; S.sphere4 = st.sphere4.p;
     S.pairs = st.pairs.p;
@@ -1951,7 +1954,7 @@ int dfpt_render(dfpt_handle* h, int32_t passes) {
     if (h->counting) CUDA_TRY(cudaMemsetAsync(h->stats.p, 0, 6 * sizeof(unsigned long long), h->stream));
     if (passes == 0) return DFPT_OK;
     h->events_used = 0;
-    refresh_packed(h);
+    refresh_walk(h);
     {
         int r = ensure_shadow_capacity(h);
         if (!r) r = pass_shadow_sort_prepare(h);
@@ -2126,7 +2129,7 @@ int dfpt_diff_backward(dfpt_handle* h, const float* dloss_dimage, double* grad_a
     for (size_t i = 0; i < n; ++i) w[i] = make_float4(dloss_dimage[3 * i], dloss_dimage[3 * i + 1], dloss_dimage[3 * i + 2], 0.0f);
     CUDA_TRY(upload(h->diff_dldi, w, h->stream));
     CUDA_TRY(cudaMemsetAsync(h->diff_rows.p, 0, h->diff_rows.n * sizeof(double), h->stream));
-    refresh_packed(h);
+    refresh_walk(h);
     // Replay the forward's passes: same pass indices, so the same RNG streams.
     const int pass0 = h->diff_pass0;
     if (h->diff_spp >= 2 && wide_eligible(h) && h->wide.b_shade_adj) {

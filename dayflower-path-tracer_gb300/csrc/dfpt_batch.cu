@@ -209,8 +209,13 @@ int batch_prepare(dfpt_batch* b) {
     b->ks.occupancy(b->sms, c.grid, c.grid_trace, c.grid_simple);
     c.trace_config = b->trace_config;
     c.grid_trace = b->ks.trace_grid(b->trace_config, b->sms);
-    c.packed = true;  // one launch walks every scene's rays
-    for (const auto& st : b->stores) c.packed = c.packed && st->scene.use_pairs == 3;
+    // One launch walks every scene's rays; the packed pair walk takes scenes without meshes too.
+    bool packed = true, flat = true;
+    for (const auto& st : b->stores) {
+        packed = packed && (st->scene.use_pairs == 3 || st->scene.flat);
+        flat = flat && st->scene.flat;
+    }
+    c.walk = flat ? 7 : packed ? 6 : 0;
     b->ctx_shadow = c;
     b->ctx_shadow.pass = &b->pass_shadow;
     return DFPT_OK;

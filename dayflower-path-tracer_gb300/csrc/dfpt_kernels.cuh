@@ -786,6 +786,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(DevScene S0, const DevPar
             },
             st);
         warp_add_stats(P, B.stats, ANY ? 1 : 0, segs, st.nodes, st.tris);
+    } else if constexpr (V == 7) {
+        // Short walks of much the same length: no work counter to wait for.
+        for (int i = blockIdx.x * BLOCK + threadIdx.x; i < n; i += gridDim.x * BLOCK) {
+            const float4 o = __ldcs(qo + i), d = __ldcs(qd + i);
+            const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
+            const Hit h = trace_flat<ANY>(S, o.x, o.y, o.z, d.x, d.y, d.z);
+            __stcs(B.q_hit + i, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset));
+        }
     } else {
         WARP_DYNAMIC(i, n, B.counts + DFPT_COUNTS_FETCH + bounce) {
             TraceStats st{0, 0};
@@ -800,7 +808,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(DevScene S0, const DevPar
             const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
             const Hit h = trace_v<ANY, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
             if (valid) __stcs(B.q_hit + i, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset));
-            if constexpr (V != 6) warp_add_stats(P, B.stats, ANY ? 1 : 0, valid ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V < 6) warp_add_stats(P, B.stats, ANY ? 1 : 0, valid ? 1u : 0u, st.nodes, st.tris);
         }
     }
 }
@@ -1224,6 +1232,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow(DevScene S0, const DevPa
             },
             st);
         warp_add_stats(P, B.stats, 1, segs, st.nodes, st.tris);
+    } else if constexpr (V == 7) {
+        for (int i = blockIdx.x * BLOCK + threadIdx.x; i < n; i += gridDim.x * BLOCK) {
+            const float4 o = __ldcs(B.s_o + i), d = __ldcs(B.s_d + i);
+            const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
+            const Hit h = trace_flat<true>(S, o.x, o.y, o.z, d.x, d.y, d.z);
+            if (h.t >= INF - 0.0001f) unoccluded(i, o, __ldcs(B.s_c + i));
+        }
     } else {
         WARP_DYNAMIC(i, n, B.counts + DFPT_COUNTS_FETCH + DFPT_MAX_DEPTH + 1) {
             TraceStats st{0, 0};
@@ -1236,7 +1251,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow(DevScene S0, const DevPa
             const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
             const Hit h = trace_v<true, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
             if (valid && h.t >= INF - 0.0001f) unoccluded(i, o, __ldcs(B.s_c + i));
-            if constexpr (V != 6) warp_add_stats(P, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V < 6) warp_add_stats(P, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
         }
     }
 }
@@ -1273,6 +1288,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_final(DevScene S0, const DevPar
             },
             st);
         warp_add_stats(P0, B.stats, 1, segs, st.nodes, st.tris);
+    } else if constexpr (V == 7) {
+        for (int i = blockIdx.x * BLOCK + threadIdx.x; i < n; i += gridDim.x * BLOCK) {
+            const float4 o = B.q_o[qi][i], d = B.q_d[qi][i];
+            const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
+            const Hit h = trace_flat<true>(S, o.x, o.y, o.z, d.x, d.y, d.z);
+            if (!(h.t < INF)) escaped(o, d);
+        }
     } else {
         WARP_DYNAMIC(i, n, B.counts + DFPT_COUNTS_FETCH + bounce) {
             TraceStats st{0, 0};
@@ -1285,7 +1307,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_final(DevScene S0, const DevPar
             const DevScene& S = scene_of<BATCH>(S0, Q, BATCH ? __float_as_int(d.w) : 0);
             const Hit h = trace_v<true, V>(S, valid, o.x, o.y, o.z, d.x, d.y, d.z, st);
             if (valid && !(h.t < INF)) escaped(o, d);
-            if constexpr (V != 6) warp_add_stats(P0, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V < 6) warp_add_stats(P0, B.stats, 1, valid ? 1u : 0u, st.nodes, st.tris);
         }
     }
 }
@@ -1336,7 +1358,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
         {
             TraceStats st{0, 0};
             const Hit h = trace_v<false, V>(S, step, o.x, o.y, o.z, d.x, d.y, d.z, st);
-            if constexpr (V != 6) warp_add_stats(P, B.stats, 0, step ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V < 6) warp_add_stats(P, B.stats, 0, step ? 1u : 0u, st.nodes, st.tris);
             bool emit_next = false, emit_shadow = false;
             float4 no = make_float4(0, 0, 0, 0), nd = make_float4(0, 0, 0, 0);
             float4 so = make_float4(0, 0, 0, 0), sd = make_float4(0, 0, 0, 0), sc = make_float4(0, 0, 0, 0);
@@ -1366,7 +1388,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
         if (__any_sync(0xFFFFFFFFu, fin)) {
             TraceStats st{0, 0};
             const Hit h = trace_v<true, V>(S, fin, o.x, o.y, o.z, d.x, d.y, d.z, st);
-            if constexpr (V != 6) warp_add_stats(P, B.stats, 1, fin ? 1u : 0u, st.nodes, st.tris);
+            if constexpr (V < 6) warp_add_stats(P, B.stats, 1, fin ? 1u : 0u, st.nodes, st.tris);
             if (fin) {
                 if (!(h.t < INF)) {
                     const int path = __float_as_int(o.w);
@@ -1387,21 +1409,23 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
 // ---------------------------------------------------------------------------------------------
 // The per-pixel modes: ray caster, ambient occlusion, surface normals, ray tracer, ray marcher.
 
-// PACKED: the packed pair walk for every ray (nothing is counted), in a function of its own: k_simple
-// calls it from four places and needs few registers beside it (64 against 112, 8 blocks of 128 per SM
-// against 4: the 1080p ray-cast view of mesh_scene 1.80 -> 1.31 ms, ambient occlusion at 1003 x 601
-// 0.71 -> 0.50 ms with its readbacks).
-__device__ __noinline__ Hit trace_simple_packed(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz) {
-    return trace_pairs<false, 128>(S, ox, oy, oz, dx, dy, dz);
+// WALK 6 and 7: the packed pair walk or the walk of scenes without meshes for every ray (LaunchCtx::walk;
+// nothing is counted), in a function of its own: k_simple calls it from four places and needs few
+// registers beside it (64 against 112, 8 blocks of 128 per SM against 4: the 1080p ray-cast view of
+// mesh_scene 1.80 -> 1.31 ms, ambient occlusion at 1003 x 601 0.71 -> 0.50 ms with its readbacks).
+template <int WALK>
+__device__ __noinline__ Hit trace_simple_walk(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz) {
+    if constexpr (WALK == 7) return trace_flat<false>(S, ox, oy, oz, dx, dy, dz);
+    else return trace_pairs<false, 128>(S, ox, oy, oz, dx, dy, dz);
 }
-template <bool PACKED>
+template <int WALK>
 __device__ __forceinline__ Hit trace_simple(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz, TraceStats& st) {
-    if constexpr (PACKED) return trace_simple_packed(S, ox, oy, oz, dx, dy, dz);
+    if constexpr (WALK != 0) return trace_simple_walk<WALK>(S, ox, oy, oz, dx, dy, dz);
     else return trace_s(S, ox, oy, oz, dx, dy, dz, st);
 }
 
 // doShaderPhongReflectionModel0 (GRK:1962-2039), with the reference's closest-hit shadow test.
-template <bool PACKED>
+template <int WALK>
 __device__ int phong0(const DevScene& S, const DevParams& P, bool test, float px, float py, float pz, float nx, float ny, float nz,
                       float vx, float vy, float vz, float ar, float ag, float ab, TraceStats& st) {
     float r = 0.0f, g = 0.0f, b = 0.0f;
@@ -1412,7 +1436,7 @@ __device__ int phong0(const DevScene& S, const DevParams& P, bool test, float px
     const float lr = 1.0f / ll;
     const float lnx = lx * lr, lny = ly * lr, lnz = lz * lr;
     float t = INF;
-    if (test) t = trace_simple<PACKED>(S, px, py, pz, lnx, lny, lnz, st).t;
+    if (test) t = trace_simple<WALK>(S, px, py, pz, lnx, lny, lnz, st).t;
     if (t >= INF || t > l2) {
         const float ldn = lnx * nx + lny * ny + lnz * nz;
         r += ar * 0.5f * jmax(ldn, 0.0f) * 1.0f;
@@ -1445,8 +1469,8 @@ __device__ float height_rm(const DevParams& P, float x, float z) {
     return fractal2(P.g_amplitude, P.g_frequency, P.g_gain, P.g_lacunarity, P.g_octaves, x, z);
 }
 
-template <bool PACKED>
-__global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(const __grid_constant__ DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
+template <int WALK>
+__global__ void __launch_bounds__(128, WALK ? 8 : 1) k_simple(const __grid_constant__ DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
     const DevParams& P = *Pp;
     const int n = B.n_pixels;
     const uint32_t pass = (uint32_t)*B.pass_index;
@@ -1481,7 +1505,7 @@ __global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(const __grid_con
                             const float nr = 1.0f / sqrtf(nx * nx + ny * ny + nz * nz);
                             const float noise = fbm3(8.0f, 0.5f, 0.0f, 1.0f, 16, px, py, pz);
                             const float al = saturate_j(noise * 1.0f + 0.1f, 0.0f, 1.0f);
-                            const int c = phong0<PACKED>(S, P, false, px, py, pz, nx * nr, ny * nr, nz * nr, -dx, -dy, -dz, al, al, al, st);
+                            const int c = phong0<WALK>(S, P, false, px, py, pz, nx * nr, ny * nr, nz * nr, -dx, -dy, -dz, al, al, al, st);
                             cr_ = cr(c); cg_ = cg(c); cb_ = cb(c);
                             t = max_t;
                         }
@@ -1490,7 +1514,7 @@ __global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(const __grid_con
                 } else {
                     const int depth_max = mode == DFPT_RENDERER_RAY_TRACER ? 5 : 1;
                     for (int depth = 0; depth < depth_max; ++depth) {
-                        const Hit h = trace_simple<PACKED>(S, ox, oy, oz, dx, dy, dz, st);
+                        const Hit h = trace_simple<WALK>(S, ox, oy, oz, dx, dy, dz, st);
                         segs++;
                         if (depth == 0) B.primitive_offsets[i] = h.prim >= 0 ? h.prim * 3 : -1;
                         if (h.t == INF || h.prim == -1) {
@@ -1529,7 +1553,7 @@ __global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(const __grid_con
                             const float e1z = e0x * u2z + e0y * v0z + e0z * w1z;
                             const float er = rsqrt_j(e1x * e1x + e1y * e1y + e1z * e1z);
                             const float aox = s.px + w1x * 0.01f, aoy = s.py + w1y * 0.01f, aoz = s.pz + w1z * 0.01f;
-                            const float t = trace_simple<PACKED>(S, aox, aoy, aoz, e1x * er, e1y * er, e1z * er, st).t;
+                            const float t = trace_simple<WALK>(S, aox, aoy, aoz, e1x * er, e1y * er, e1z * er, st).t;
                             segs++;
                             const bool hit = t < P.ao_max_distance;
                             const float v = hit ? 1.0f : 0.0f;  // bright 1, dark 0
@@ -1546,7 +1570,7 @@ __global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(const __grid_con
                         } else {
                             ar = cr(albedo); ag = cg(albedo); ab = cb(albedo);
                         }
-                        const int c = phong0<PACKED>(S, P, true, s.px, s.py, s.pz, wx, wy, wz, -dx, -dy, -dz, ar, ag, ab, st);
+                        const int c = phong0<WALK>(S, P, true, s.px, s.py, s.pz, wx, wy, wz, -dx, -dy, -dz, ar, ag, ab, st);
                         segs++;
                         if (mode == DFPT_RENDERER_RAY_CASTER) {
                             cr_ = cr(c); cg_ = cg(c); cb_ = cb(c);
@@ -1565,7 +1589,7 @@ __global__ void __launch_bounds__(128, PACKED ? 8 : 1) k_simple(const __grid_con
             B.radiance[PSI(i)] = make_float4(cr_, cg_, cb_, 0.0f);
             B.rng[i] = rng.state;
         }
-        if constexpr (!PACKED) warp_add_stats(P, B.stats, 0, segs, st.nodes, st.tris);
+        if constexpr (WALK == 0) warp_add_stats(P, B.stats, 0, segs, st.nodes, st.tris);
     }
 }
 
@@ -2042,6 +2066,9 @@ __global__ void k_init_tables(const int* perm256, const float* grad36) {
 #define BATCH_SCENE(c) DevScene{}
 #endif
 
+// Resident blocks of 256 for scenes without meshes: 4 (48-56 registers, no spills); 5, 6 and 8 measured
+// 0.46, 0.50 and 0.76 ms against 0.44 for the closest hits of 64 passes of sphere_scene.
+#define DFPT_FLAT_MINB 4
 // A grid of every block of `kernel` that the current device holds at once.
 template <class Kernel>
 static int resident_grid(Kernel kernel, int block) {
@@ -2065,11 +2092,15 @@ struct TraceCfg {
 #endif
     }
 #ifndef DFPT_ONE_SCENE
-    // Configurations of the compact pair walk (V 5) launch the packed pair walk (6) where it may run.
+    // Configurations of the compact pair walk (V 5) launch the walk that LaunchCtx::walk names.
     static void closest(const LaunchCtx& c, int bounce) {
         if constexpr (V == 5) {
-            if (c.packed) {
+            if (c.walk == 6) {
                 k_trace<false, false, 6, BLOCK, MINB><<<resident_grid(k_trace<false, false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                return;
+            }
+            if (c.walk == 7) {
+                k_trace<false, false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_trace<false, false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
                 return;
             }
         }
@@ -2077,8 +2108,12 @@ struct TraceCfg {
     }
     static void shadow(const LaunchCtx& c, int bounce) {
         if constexpr (V == 5) {
-            if (c.packed) {
+            if (c.walk == 6) {
                 k_shadow<false, 6, BLOCK, MINB><<<resident_grid(k_shadow<false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                return;
+            }
+            if (c.walk == 7) {
+                k_shadow<false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_shadow<false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
                 return;
             }
         }
@@ -2086,8 +2121,12 @@ struct TraceCfg {
     }
     static void final_(const LaunchCtx& c, int bounce) {
         if constexpr (V == 5) {
-            if (c.packed) {
+            if (c.walk == 6) {
                 k_final<false, 6, BLOCK, MINB><<<resident_grid(k_final<false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                return;
+            }
+            if (c.walk == 7) {
+                k_final<false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_final<false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
                 return;
             }
         }
@@ -2107,8 +2146,12 @@ struct TraceCfg {
     template <int TB>
     static void tail_t(const LaunchCtx& c, int b0, int nb) {
         if constexpr (TVV == 5) {
-            if (c.packed) {
+            if (c.walk == 6) {
                 k_tail<6, 256, TB><<<resident_grid(k_tail<6, 256, TB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
+                return;
+            }
+            if (c.walk == 7) {
+                k_tail<7, 256, TB><<<resident_grid(k_tail<7, 256, TB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
                 return;
             }
         }
@@ -2129,8 +2172,12 @@ struct TraceCfg {
     static constexpr int BV = V == 2 ? 1 : V;
     static void b_closest(const LaunchCtx& c, int bounce) {
         if constexpr (BV == 5) {
-            if (c.packed) {
+            if (c.walk == 6) {
                 k_trace<true, false, 6, BLOCK, MINB><<<resident_grid(k_trace<true, false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                return;
+            }
+            if (c.walk == 7) {
+                k_trace<true, false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_trace<true, false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
                 return;
             }
         }
@@ -2138,8 +2185,12 @@ struct TraceCfg {
     }
     static void b_shadow(const LaunchCtx& c, int bounce) {
         if constexpr (BV == 5) {
-            if (c.packed) {
+            if (c.walk == 6) {
                 k_shadow<true, 6, BLOCK, MINB><<<resident_grid(k_shadow<true, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                return;
+            }
+            if (c.walk == 7) {
+                k_shadow<true, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_shadow<true, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
                 return;
             }
         }
@@ -2147,8 +2198,12 @@ struct TraceCfg {
     }
     static void b_final(const LaunchCtx& c, int bounce) {
         if constexpr (BV == 5) {
-            if (c.packed) {
+            if (c.walk == 6) {
                 k_final<true, 6, BLOCK, MINB><<<resident_grid(k_final<true, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                return;
+            }
+            if (c.walk == 7) {
+                k_final<true, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_final<true, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
                 return;
             }
         }
@@ -2288,8 +2343,9 @@ static void launch_diff_reduce(const LaunchCtx& c, const double* rows, int n_row
 #endif
 #ifndef DFPT_ONE_SCENE
 static void launch_simple(const LaunchCtx& c) {
-    if (c.packed) k_simple<true><<<resident_grid(k_simple<true>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
-    else k_simple<false><<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    if (c.walk == 6) k_simple<6><<<resident_grid(k_simple<6>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    else if (c.walk == 7) k_simple<7><<<resident_grid(k_simple<7>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    else k_simple<0><<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
 }
 static void launch_wireframe(const LaunchCtx& c) { k_wireframe<<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass); }
 static void launch_film(const LaunchCtx& c) { k_film<<<c.grid, 256, 0, c.stream>>>(c.params, *c.pass); }
@@ -2325,7 +2381,7 @@ static void occupancy(int sms, int& grid, int& grid_trace, int& grid_simple) {
     b3 = b1;
 #else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_shade<false>, 256, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, k_simple<false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, k_simple<0>, 128, 0);
 #endif
     grid = sms * (b1 > 0 ? b1 : 1);
     grid_trace = trace_grid(0, sms);

@@ -17,7 +17,9 @@ struct LaunchCtx {
     int trace_config;  // index into the kernel set's traversal configurations
     const DevBatch* batch = nullptr;  // batch launches only
     int tail_blocks = 2;              // resident blocks per SM the tail kernel is compiled for (2-4)
-    bool packed = false;              // configurations 16 and 17 and the per-pixel modes may take the packed pair walk
+    // What configurations 16 and 17 and the per-pixel modes walk with: 6 the packed pair walk, 7 scenes
+    // without meshes, 0 the configuration's own (counting) walk.
+    int walk = 0;
 };
 
 struct KernelSet {

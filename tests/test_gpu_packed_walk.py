@@ -6,7 +6,8 @@ tracer's films agree to the rounding that float atomics leave (rtol 1e-5, as for
 of walk orders). Trees at the edges: a root that is a leaf, two leaves, chains of boxes deep enough
 to leave the shared-memory stack, as deep as the walk takes and one level deeper, boxes that do not nest (the scene
 then keeps the counting walk's order), meshes with shared and with different matrices, every
-culling mode.
+culling mode. Scenes without meshes take a walk of their own (the culling BVH nearer child first): from
+no bounded primitive to 90, spheres and triangles, and pairs of them in the same place.
 """
 import numpy as np
 import pytest
@@ -75,9 +76,37 @@ def _chain(compiled):
     return compiled
 
 
+def _flat_scene(count, shape, duplicates=False):
+    """`count` spheres or triangle primitives over a plane and no mesh; duplicates: every second one
+    where the one before it is, with another material (equal distances: the first one counts)."""
+    from dfpt import scene as sc, synthetic
+
+    rng = np.random.default_rng(count)
+    b = sc.SceneBuilder()
+    black = b.constant(0, 0, 0)
+    b.primitive(b.plane((0, -1.5, 0), (0, -1.5, 1), (1, -1.5, 0)), b.surface(sc.LAMBERTIAN, b.constant(0.5, 0.5, 0.5), black, black))
+    sphere = b.sphere((0, 0, 0), 0.35)
+    position = np.zeros(3)
+    for k in range(count):
+        if not (duplicates and k % 2):
+            position = rng.uniform((-2.5, -1.5, -3.0), (2.5, 1.8, 1.5))
+        surf = b.surface((sc.LAMBERTIAN, sc.GLASS, sc.PHONG, sc.CLEAR_COAT)[k % 4], b.constant(*rng.uniform(0.3, 0.9, 3)), black, black)
+        if shape == "sphere":
+            b.primitive(sphere, surf, position=tuple(float(v) for v in position))
+        else:
+            v = position + np.asarray([(0.0, 0.5, 0.0), (-0.5, -0.3, 0.1), (0.5, -0.4, -0.2)])
+            n = synthetic.vertex_normals(v, np.arange(3).reshape(1, 3))
+            b.primitive(b.mesh(v, [[0, 1, 2]], n, np.zeros((3, 2)), synthetic.tangents_for(n), as_mesh=False), surf)
+    b.camera((0.3, 0.7, 6.0), (0.05, 0.0, 0.0), 60.0, (72, 56))
+    return b.compile("flat"), sc.SkyState((0.5, 0.7, 0.4), 2.5), dict(renderer_type=2, pt_ray_depth_maximum=5, pt_ray_depth_russian_roulette=3, tone_mapper_type=2)
+
+
 def _scene(name):
     from dfpt import synthetic
 
+    if name.startswith("flat_"):
+        _, shape, count = name.split("_")[:3]
+        return _flat_scene(int(count), shape, name.endswith("twice"))
     if name == "sphere":
         pos, idx, _, _, _ = synthetic.displaced_icosphere(6, 0.2, 4, radius=1.7)
         return _mesh_scene(pos, idx)
@@ -112,10 +141,12 @@ def _render(compiled, sky, params, counting, culling, passes):
     return out
 
 
-@pytest.mark.parametrize("name", ["one", "two", "five", "sphere", "chain", "deepest", "too_deep", "not_nested", "shared_matrix", "own_matrices", "many"])
+@pytest.mark.parametrize("name", ["one", "two", "five", "sphere", "chain", "deepest", "too_deep", "not_nested", "shared_matrix", "own_matrices", "many",
+                                  "flat_sphere_0", "flat_sphere_3", "flat_sphere_8", "flat_sphere_90", "flat_sphere_90_twice", "flat_triangle_30",
+                                  "flat_triangle_30_twice"])
 def test_packed_walk_equals_counting_walk(name):
     compiled, sky, params = _scene(name)
-    for culling in ((0, 1, 2) if name == "many" else (0,)):
+    for culling in ((0, 1, 2) if compiled.primitive_count > 8 else (0,)):
         for renderer in (3, 1, 5, 6):
             a, b = (_render(compiled, sky, dict(params, renderer_type=renderer), c, culling, 1) for c in (False, True))
             assert (a[3] >= 0).any(), "no ray hits the scene"
