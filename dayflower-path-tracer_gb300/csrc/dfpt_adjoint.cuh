@@ -210,6 +210,13 @@ __device__ void sun_rim_tan(const DevScene& S, const DevParams& P, uint32_t pixe
 
 // Per-block gradient accumulation: per-primitive entries in shared memory (float, one launch) when
 // they fit, else straight into row 0 with double atomics; the four sky entries in registers.
+//
+// A vertex's seven entries are gathered in registers and added by the warp together: lanes of one
+// primitive sum theirs with shuffles and one lane adds the sums. A float atomic on shared memory is
+// a compare-and-swap loop, and a wave's neighbouring lanes mostly hit one primitive (at bounce 0 the
+// samples of one or two pixels), so lane by lane the loops ran up to 32 times for each entry: the
+// backward of 16 passes at 512 x 512 over 257 primitives took 5.8 ms, 4.0 now.
+// Groups of fewer than 4 lanes add on their own.
 struct GradAcc {
     float* sh;     // shared [P * 7] or null
     double* row;   // this block's row (shared mode) / row 0 (atomic mode)
@@ -217,6 +224,26 @@ struct GradAcc {
         if (v == 0.0f) return;
         if (sh) atomicAdd(sh + prim * DFPT_DIFF_PER_PRIM + k, v);
         else atomicAdd(row + prim * DFPT_DIFF_PER_PRIM + k, (double)v);
+    }
+    // All 32 lanes call it; prim < 0: no vertex.
+    __device__ __forceinline__ void add_warp(int prim, const float g[DFPT_DIFF_PER_PRIM]) {
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, prim);
+        const int lane = threadIdx.x & 31;
+        const bool grouped = prim >= 0 && __popc(same) >= 4;
+        if (prim >= 0 && !grouped)
+            for (int k = 0; k < DFPT_DIFF_PER_PRIM; ++k) add(prim, k, g[k]);
+        unsigned todo = __ballot_sync(0xFFFFFFFFu, grouped);
+        while (todo) {
+            const int leader = __ffs(todo) - 1;
+            const unsigned group = __shfl_sync(0xFFFFFFFFu, same, leader);
+            const bool in = (group >> lane) & 1u;
+            for (int k = 0; k < DFPT_DIFF_PER_PRIM; ++k) {
+                float v = in ? g[k] : 0.0f;
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+                if (lane == leader) add(prim, k, v);
+            }
+            todo &= ~group;
+        }
     }
 };
 
@@ -268,6 +295,8 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
     GRID_STRIDE_UNIFORM(i, n) {
         bool emit_next = false;
         float4 no = make_float4(0, 0, 0, 0), nd = make_float4(0, 0, 0, 0);
+        int vertex = -1;  // its primitive, and what it adds to the primitive's entries
+        float g[DFPT_DIFF_PER_PRIM] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         if (i < n) {
             const float4 o4 = B.q_o[qi][i], d4 = B.q_d[qi][i];
             const int path = __float_as_int(o4.w);
@@ -314,9 +343,10 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                 diff_surface(P, h.prim, ar, ag, ab, er, eg, eb, exponent);
                 // Emission.
                 Lu.x += T.x * er; Lu.y += T.y * eg; Lu.z += T.z * eb;
-                acc.add(h.prim, 3, w.x * T.x);
-                acc.add(h.prim, 4, w.y * T.y);
-                acc.add(h.prim, 5, w.z * T.z);
+                vertex = h.prim;
+                g[3] = w.x * T.x;
+                g[4] = w.y * T.y;
+                g[5] = w.z * T.z;
                 // Sun sample (same draws as the forward; visibility from the forward's bits).
                 if ((material == DFPT_MATERIAL_CLEAR_COAT || material == DFPT_MATERIAL_LAMBERTIAN || material == DFPT_MATERIAL_PHONG) &&
                     P.sun_active == 1) {
@@ -328,9 +358,9 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                     if (sun_sample(P, s.px, s.py, s.pz, wx, wy, wz, u, v, lx, ly, lz, dot1) && seen) {
                         const float k = dot1 * INV_PI;
                         Lu.x += T.x * (ar * 1.0f * k); Lu.y += T.y * (ag * 1.0f * k); Lu.z += T.z * (ab * 1.0f * k);
-                        acc.add(h.prim, 0, w.x * T.x * tr * k);
-                        acc.add(h.prim, 1, w.y * T.y * tg * k);
-                        acc.add(h.prim, 2, w.z * T.z * tb * k);
+                        g[0] = w.x * T.x * tr * k;
+                        g[1] = w.y * T.y * tg * k;
+                        g[2] = w.z * T.z * tb * k;
                         g_forward = c * dot1;
                     }
                     sun_rim_tan(S, P, pixel, pass, bounce, s.px, s.py, s.pz, wx, wy, wz, c, g_forward, gsky);
@@ -352,12 +382,12 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                     // Radiance of the later vertices (every term carries this vertex's factors).
                     const float lr = Lt.x - Lu.x, lg = Lt.y - Lu.y, lb = Lt.z - Lu.z;
                     if (sct.albedo) {
-                        if (a0r != 0.0f) acc.add(h.prim, 0, w.x * lr * tr / a0r);
-                        if (a0g != 0.0f) acc.add(h.prim, 1, w.y * lg * tg / a0g);
-                        if (a0b != 0.0f) acc.add(h.prim, 2, w.z * lb * tb / a0b);
+                        if (a0r != 0.0f) g[0] += w.x * lr * tr / a0r;
+                        if (a0g != 0.0f) g[1] += w.y * lg * tg / a0g;
+                        if (a0b != 0.0f) g[2] += w.z * lb * tb / a0b;
                     }
                     if (material == DFPT_MATERIAL_PHONG && sct.phong_ct > 0.0f)
-                        acc.add(h.prim, 6, (w.x * lr + w.y * lg + w.z * lb) * (1.0f / (exponent + 1.0f) + logf(sct.phong_ct)));
+                        g[6] = (w.x * lr + w.y * lg + w.z * lb) * (1.0f / (exponent + 1.0f) + logf(sct.phong_ct));
                     emit_next = true;
                     no = make_float4(sct.o.x, sct.o.y, sct.o.z, __int_as_float(path));
                     nd = make_float4(sct.d.x, sct.d.y, sct.d.z, 0.0f);
@@ -367,6 +397,7 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                 B.rng[path] = rng.state;
             }
         }
+        acc.add_warp(vertex, g);
         const int slot = warp_push(B.counts + bounce + 1, emit_next);
         if (slot >= 0) {
             B.q_o[qi ^ 1][slot] = no;
@@ -413,11 +444,19 @@ __global__ void __launch_bounds__(256) k_final_adj(DevScene S, const DevParams* 
     grad_end(nullptr, B.diff_rows + (size_t)blockIdx.x * B.diff_row_len, n_prim_entries, gsky, red);
 }
 
-// Sums the per-block rows into out[row_len].
-__global__ void k_diff_reduce(const double* __restrict__ rows, int n_rows, int row_len, double* __restrict__ out) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < row_len; k += gridDim.x * blockDim.x) {
-        double t = 0.0;
-        for (int r = 0; r < n_rows; ++r) t += rows[(size_t)r * row_len + k];
+// Sums the per-block rows into out[row_len]: a block takes 32 entries, its 8 warps every eighth row each
+// (one thread per entry walked all rows one after the other: 80 us for 456 rows of 1,803, now 11).
+__global__ void __launch_bounds__(256) k_diff_reduce(const double* __restrict__ rows, int n_rows, int row_len, double* __restrict__ out) {
+    __shared__ double part[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = blockIdx.x * 32 + lane;
+    double t = 0.0;
+    if (k < row_len)
+        for (int r = w; r < n_rows; r += 8) t += rows[(size_t)r * row_len + k];
+    part[w][lane] = t;
+    __syncthreads();
+    if (w == 0 && k < row_len) {
+        for (int j = 1; j < 8; ++j) t += part[j][lane];
         out[k] = t;
     }
 }

@@ -5,6 +5,8 @@
 // AbstractImageKernel.java (src/main/java/org/dayflower/pathtracer/kernel/).
 #pragma once
 
+#include <algorithm>
+
 #include "dfpt_device.cuh"
 #include "dfpt_launch.h"
 
@@ -2071,11 +2073,11 @@ __global__ void k_init_tables(const int* perm256, const float* grad36) {
 #define DFPT_FLAT_MINB 4
 // A grid of every block of `kernel` that the current device holds at once.
 template <class Kernel>
-static int resident_grid(Kernel kernel, int block) {
+static int resident_grid(Kernel kernel, int block, size_t dynamic_shared = 0) {
     int dev = 0, sms = 0, b = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, block, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, block, dynamic_shared);
     return (sms > 0 ? sms : 1) * (b > 0 ? b : 1);
 }
 
@@ -2322,8 +2324,10 @@ template <bool BATCH>
 static void launch_shade_adj_t(const LaunchCtx& c, int bounce) {
     const DevBatch Q = BATCH ? *c.batch : DevBatch{};
     const size_t bytes = (size_t)c.scene->primitive_count * DFPT_DIFF_PER_PRIM * sizeof(float);
-    if (bytes <= 44 * 1024) k_shade_adj<BATCH, true><<<c.grid, 256, bytes, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
-    else k_shade_adj<BATCH, false><<<c.grid, 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
+    // One row per block of c.grid blocks; no more than are resident (at 128 registers 2 per SM, where
+    // c.grid's 3 left a second round half empty).
+    if (bytes <= 44 * 1024) k_shade_adj<BATCH, true><<<std::min(c.grid, resident_grid(k_shade_adj<BATCH, true>, 256, bytes)), 256, bytes, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
+    else k_shade_adj<BATCH, false><<<std::min(c.grid, resident_grid(k_shade_adj<BATCH, false>, 256)), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
 }
 template <bool BATCH>
 static void launch_final_adj_t(const LaunchCtx& c, int bounce) {
@@ -2338,7 +2342,7 @@ static void launch_final_adj(const LaunchCtx& c, int bounce) { launch_final_adj_
 static void launch_b_shade_adj(const LaunchCtx& c, int bounce) { launch_shade_adj_t<true>(c, bounce); }
 static void launch_b_final_adj(const LaunchCtx& c, int bounce) { launch_final_adj_t<true>(c, bounce); }
 static void launch_diff_reduce(const LaunchCtx& c, const double* rows, int n_rows, int row_len, double* out) {
-    k_diff_reduce<<<(row_len + 255) / 256, 256, 0, c.stream>>>(rows, n_rows, row_len, out);
+    k_diff_reduce<<<(row_len + 31) / 32, 256, 0, c.stream>>>(rows, n_rows, row_len, out);
 }
 #endif
 #ifndef DFPT_ONE_SCENE
