@@ -865,6 +865,8 @@ int wide_prepare(dfpt_handle* h) {
     B.sort_count = h->w_sort_bins.p + DFPT_SORT_BINS;
     B.sort_count_shadow = h->shadow_sort ? h->w_sort_bins.p + 2 * DFPT_SORT_BINS : nullptr;  // null: shadow rays unbinned
     B.sort_partials = h->w_sort_bins.p + 3 * DFPT_SORT_BINS;
+    B.sort_ray_bits = sort_bits(h->wide_capacity, DFPT_RAY_DIRS, 4, DFPT_RAY_CELL_BITS);
+    B.sort_shadow_bits = sort_bits(h->wide_capacity, 1, 6, DFPT_SHADOW_CELL_BITS);
     if (h->diff_on) {
         // The differentiable forward / replay: visibility bits per slot, the per-sample records.
         if (!h->w_vis.p) CUDA_TRY(h->w_vis.alloc((size_t)h->wide_capacity));
@@ -1062,6 +1064,7 @@ int pass_shadow_sort_prepare(dfpt_handle* h) {
     B.sort_count_shadow = shadow_counts;
     B.sort_partials = h->p_sort_bins.p + 3 * DFPT_SORT_BINS;
     B.sort_ray_bits = h->pass_ray_sort;
+    B.sort_shadow_bits = sort_bits(h->n_pixels, 1, 6, DFPT_SHADOW_CELL_BITS);
     h->pass_shadow2 = B;
     h->pass_shadow2.s_o = h->p_s2_o.p;
     h->pass_shadow2.s_d = h->p_s2_d.p;

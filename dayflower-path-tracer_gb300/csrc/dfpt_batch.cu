@@ -182,6 +182,13 @@ int batch_prepare(dfpt_batch* b) {
     B.sort_count = b->sort_bins.p ? b->sort_bins.p + DFPT_SORT_BINS : nullptr;
     B.sort_count_shadow = b->sort_bins.p ? b->sort_bins.p + 2 * DFPT_SORT_BINS : nullptr;
     B.sort_partials = b->sort_bins.p ? b->sort_bins.p + 3 * DFPT_SORT_BINS : nullptr;
+    if (b->stores.size() > 1) {
+        B.sort_ray_bits = sort_bits(b->capacity, 8 * 128, 4, 12);
+        B.sort_shadow_bits = sort_bits(b->capacity, 8, 6, 18);
+    } else {
+        B.sort_ray_bits = sort_bits(b->capacity, DFPT_RAY_DIRS, 4, DFPT_RAY_CELL_BITS);
+        B.sort_shadow_bits = sort_bits(b->capacity, 1, 6, DFPT_SHADOW_CELL_BITS);
+    }
     b->pass_shadow = B;
     if (B.sorted_queues) {
         b->pass_shadow.s_o = b->s2_o.p;

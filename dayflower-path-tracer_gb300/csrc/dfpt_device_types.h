@@ -167,32 +167,31 @@ struct DevPass {
     int* sort_count;           // DFPT_SORT_BINS ray counts of the next bounce; zero at rest (the scan clears them)
     int* sort_count_shadow;    // the same for the sun shadow rays
     int* sort_partials;        // DFPT_SORT_CHUNKS chunk sums of the scan
-    int sort_ray_bits;         // plain passes: origin-grid bits of the bounce rays' bins (plain_ray_bin)
+    int sort_ray_bits;         // origin-grid bits of the bounce rays' bins
+    int sort_shadow_bits;      // and of the shadow rays'
 };
-// Bins: waves of several scenes use 3 bits of scene (within a wave) x a 6 x 4 x 4 cube-map
-// direction bin (7 bits) x 12 bits of origin cell (bounce rays), or 3 bits of scene x 18 bits of
-// cell (shadow rays); waves of one scene use a direction bin (DFPT_RAY_DIR_RES) over an origin grid
-// of DFPT_RAY_CELL_BITS bits (bounce rays) or a grid of DFPT_SHADOW_CELL_BITS bits (shadow rays),
-// multiples of 3 (an equal split over the axes). Every key stays below DFPT_SORT_BINS (2^22 with
-// these settings). The scan runs over DFPT_SORT_CHUNKS chunks of 1024 bins.
-#ifndef DFPT_RAY_CELL_BITS
+// Bins. One scene: a bounce ray's bin is one of 96 cube-map directions (6 x 4 x 4) over an origin grid
+// of sort_ray_bits bits, a shadow ray's the cell of a grid of sort_shadow_bits bits (multiples of 3: an
+// equal split over the axes). Waves of several scenes: 3 bits of the scene's place in the wave above
+// either, the direction then in 7 bits. The grids follow the slots of a launch (sort_bits below), up
+// to DFPT_RAY_CELL_BITS and DFPT_SHADOW_CELL_BITS (12 and 18 with several scenes); every key stays
+// below DFPT_SORT_BINS. The scan runs over chunks of 1024 bins.
 #define DFPT_RAY_CELL_BITS 15
-#endif
-#ifndef DFPT_SHADOW_CELL_BITS
 #define DFPT_SHADOW_CELL_BITS 21
-#endif
-#ifndef DFPT_RAY_DIR_RES
-#define DFPT_RAY_DIR_RES 4  // 0: direction octant (3 bits); n: cube-map bins, 6 x n x n directions
-#endif
-#ifndef DFPT_BATCH_DIR_BINS
-#define DFPT_BATCH_DIR_BINS 1  // waves of several scenes: 1 cube-map 6 x 4 x 4 direction bins, 0 the octant
-#endif
-#define DFPT_RAY_DIR_COUNT (DFPT_RAY_DIR_RES ? 6 * DFPT_RAY_DIR_RES * DFPT_RAY_DIR_RES : 8)
-#define DFPT_RAY_DIR_BITS (DFPT_RAY_DIR_COUNT <= 8 ? 3 : DFPT_RAY_DIR_COUNT <= 16 ? 4 : DFPT_RAY_DIR_COUNT <= 32 ? 5 : \
-                           DFPT_RAY_DIR_COUNT <= 64 ? 6 : DFPT_RAY_DIR_COUNT <= 128 ? 7 : DFPT_RAY_DIR_COUNT <= 256 ? 8 : 9)
-#define DFPT_SORT_BITS (DFPT_RAY_CELL_BITS + DFPT_RAY_DIR_BITS > DFPT_SHADOW_CELL_BITS ? DFPT_RAY_CELL_BITS + DFPT_RAY_DIR_BITS : DFPT_SHADOW_CELL_BITS)
-#define DFPT_SORT_BINS (1 << (DFPT_SORT_BITS < 22 ? 22 : DFPT_SORT_BITS))  // several scenes: up to 22 bits
+#define DFPT_RAY_DIRS 96
+#define DFPT_SORT_BINS (1 << 22)
 #define DFPT_SORT_CHUNKS (DFPT_SORT_BINS / 1024)
+
+// The grid's bits for bins of `per_cell` keys a cell: as fine as leaves `rays` rays a bin when each of
+// `slots` slots emits one, at least 3, at most `most`. The scan reads and writes every bin, so bins that
+// most rays of a bounce have to themselves cost more than their order gives: with 2^21 and 2^22 bins
+// whatever the wave, binning took 1.9 ms of the 10.0 ms that 19 passes of mesh_scene at 641 x 479 took
+// (2.4 M slots a wave), and 25 of the 150 us of a 256 x 256 frame.
+inline int sort_bits(long long slots, int per_cell, int rays, int most) {
+    int bits = most;
+    while (bits > 3 && ((long long)per_cell << bits) * rays > slots) bits -= 3;
+    return bits;
+}
 
 // Many scenes rendered by one set of launches. Every scene's samples form one global sequence
 // (scene-major, then sample, then pixel); a wave takes `capacity` consecutive samples of it, one

@@ -954,7 +954,6 @@ __device__ __forceinline__ Scatter scatter(const Surf& s, int material, float wx
 // way, so a warp of them walks much the same nodes. Only the processing order changes: every ray
 // keeps its path id and its own result. Keys stay below DFPT_SORT_BINS.
 __device__ __forceinline__ int wave_first_scene(const DevBatch& Q) { return (int)Q.wave_tab[0]; }
-__device__ __forceinline__ int cell_bits(const DevScene& S, float4 o, int bits);
 // Cube-map direction bin: the major axis and its sign, the two minor components over the face in
 // N steps each (6 N^2 values).
 template <int N>
@@ -967,74 +966,44 @@ __device__ __forceinline__ int cube_dir_bin(float4 d) {
     const int iu = min(N - 1, max(0, (int)(u * r + 0.5f * N))), iv = min(N - 1, max(0, (int)(v * r + 0.5f * N)));
     return ((major * 2 + (m < 0.0f ? 1 : 0)) * N + iu) * N + iv;
 }
-__device__ __forceinline__ int ray_bin_in_wave(const DevBatch& Q, int first, float4 o, float4 d) {
-    const int sid = __float_as_int(d.w);
-    if (Q.n_scenes == 1) {
-#if DFPT_RAY_DIR_RES
-        // One scene in the wave: a cube-map direction bin over the origin grid.
-        return (cube_dir_bin<DFPT_RAY_DIR_RES>(d) << DFPT_RAY_CELL_BITS) | cell_bits(Q.scenes[sid], o, DFPT_RAY_CELL_BITS);
-#else
-        // One scene in the wave: no scene bits; the octant over the origin grid.
-        const int oct = (d.x < 0.0f ? 1 : 0) | (d.y < 0.0f ? 2 : 0) | (d.z < 0.0f ? 4 : 0);
-        return (oct << DFPT_RAY_CELL_BITS) | cell_bits(Q.scenes[sid], o, DFPT_RAY_CELL_BITS);
-#endif
+
+// Origin cell over the scene bounds with `bits` bits in all (a multiple of 3, at most 21): the cell of
+// the 128^3 grid, its axis bits interleaved from the least significant up, without the lowest ones.
+__device__ __forceinline__ int spread3(int x) {  // 7 bits, two zeros after each
+    x = (x | (x << 8)) & 0x0000F00F;
+    x = (x | (x << 4)) & 0x000C30C3;
+    return (x | (x << 2)) & 0x00249249;
+}
+__device__ __forceinline__ int cell_bits(const DevScene& S, float4 o, int bits) {
+    const float lo[3] = {S.bounds_lo.x, S.bounds_lo.y, S.bounds_lo.z};
+    const float hi[3] = {S.bounds_hi.x, S.bounds_hi.y, S.bounds_hi.z};
+    const float p[3] = {o.x, o.y, o.z};
+    int c[3];
+    for (int a = 0; a < 3; ++a) {
+        const float u = (p[a] - lo[a]) * (128.0f * __frcp_rn(hi[a] - lo[a]));  // any monotone mapping bins alike
+        c[a] = u >= 0.0f ? (u < 127.0f ? (int)u : 127) : 0;
     }
-#if DFPT_BATCH_DIR_BINS
-    // Several scenes: 3 bits of the scene's place in the wave over a 6 x 4 x 4 direction bin
-    // (7 bits) and a 16^3 grid.
-    return (((sid - first) & 7) << 19) | (cube_dir_bin<4>(d) << 12) | cell_bits(Q.scenes[sid], o, 12);
-#else
-    // Several scenes: 3 bits of the scene's place in the wave over the octant and a 32^3 grid.
-    const int oct = (d.x < 0.0f ? 1 : 0) | (d.y < 0.0f ? 2 : 0) | (d.z < 0.0f ? 4 : 0);
-    return (((sid - first) & 7) << 18) | (oct << 15) | cell_bits(Q.scenes[sid], o, 15);
-#endif
+    return (spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2)) >> (21 - bits);
 }
 
-// A plain pass's bounce ray: a 6 x 4 x 4 cube-map direction bin over an origin grid of `bits`
-// bits (a multiple of 3, at most 15).
 __device__ __forceinline__ int plain_ray_bin(const DevScene& S, float4 o, float4 d, int bits) {
     return (cube_dir_bin<4>(d) << bits) | cell_bits(S, o, bits);
+}
+__device__ __forceinline__ int ray_bin_in_wave(const DevBatch& Q, int first, float4 o, float4 d, int bits) {
+    const int sid = __float_as_int(d.w);
+    const int bin = plain_ray_bin(Q.scenes[sid], o, d, bits);
+    return Q.n_scenes == 1 ? bin : (((sid - first) & 7) << (bits + 7)) | bin;
+}
+__device__ __forceinline__ int shadow_bin_in_wave(const DevBatch& Q, int first, float4 o, float4 d, int bits) {
+    const int sid = __float_as_int(d.w);
+    const int bin = cell_bits(Q.scenes[sid], o, bits);
+    return Q.n_scenes == 1 ? bin : (((sid - first) & 7) << bits) | bin;
 }
 
 // Bin counts with one atomic per distinct bin of a warp.
 __device__ __forceinline__ void bin_count(int* bins, int key) {
     const unsigned same = __match_any_sync(0xFFFFFFFFu, key);
     if (key >= 0 && (int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(bins + key, __popc(same));
-}
-
-
-// Origin cell over the scene bounds with `bits` bits in all (at most 24: bits / 3 per axis, the
-// remainder to the axes of largest extent), axis bits interleaved from the least significant up.
-__device__ __forceinline__ int cell_bits(const DevScene& S, float4 o, int bits) {
-    const float lo[3] = {S.bounds_lo.x, S.bounds_lo.y, S.bounds_lo.z};
-    const float hi[3] = {S.bounds_hi.x, S.bounds_hi.y, S.bounds_hi.z};
-    const float p[3] = {o.x, o.y, o.z};
-    const float ext[3] = {hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]};
-    int nb[3] = {bits / 3, bits / 3, bits / 3};
-    int extra = bits - 3 * (bits / 3);
-    // The smallest axis gets no extra bit; with 2 extra, the other two get one each.
-    const int small = ext[0] <= ext[1] && ext[0] <= ext[2] ? 0 : ext[1] <= ext[2] ? 1 : 2;
-    for (int a = 0; a < 3 && extra > 0; ++a)
-        if (a != small || extra == 3) { ++nb[a]; --extra; }
-    int c[3];
-    for (int a = 0; a < 3; ++a) {
-        const float n = (float)(1 << nb[a]);
-        const float u = (p[a] - lo[a]) * (n * __frcp_rn(ext[a]));  // any monotone mapping bins alike
-        c[a] = u >= 0.0f ? (u < n - 1.0f ? (int)u : (1 << nb[a]) - 1) : 0;
-    }
-    int cell = 0, k = 0;
-    for (int b = 0; b < 8; ++b)
-        for (int a = 0; a < 3; ++a)
-            if (b < nb[a]) cell |= ((c[a] >> b) & 1) << k++;
-    return cell;
-}
-
-__device__ __forceinline__ int shadow_bin_in_wave(const DevBatch& Q, int first, float4 o, float4 d) {
-    const int sid = __float_as_int(d.w);
-    // One scene in the wave: the origin grid alone.
-    if (Q.n_scenes == 1) return cell_bits(Q.scenes[sid], o, DFPT_SHADOW_CELL_BITS);
-    // Several scenes: 3 bits of the scene's place in the wave over a 64^3 grid.
-    return (((sid - first) & 7) << 18) | cell_bits(Q.scenes[sid], o, 18);
 }
 
 // One ray's shading at one bounce: miss -> sky; hit -> emission, sun sample (a shadow ray), Russian
@@ -1184,14 +1153,14 @@ __global__ void __launch_bounds__(256, DFPT_SHADE_MINB) k_shade(DevScene S0, con
             // Ray binning: the histograms of the next bounce's rays and of the shadow rays.
             if (B.sorted_queues) {
                 const int first = wave_first_scene(Q);
-                bin_count(B.sort_count, emit_next ? ray_bin_in_wave(Q, first, no, nd) : -1);
-                if (B.sort_count_shadow) bin_count(B.sort_count_shadow, emit_shadow ? shadow_bin_in_wave(Q, first, so, sd) : -1);
+                bin_count(B.sort_count, emit_next ? ray_bin_in_wave(Q, first, no, nd, B.sort_ray_bits) : -1);
+                if (B.sort_count_shadow) bin_count(B.sort_count_shadow, emit_shadow ? shadow_bin_in_wave(Q, first, so, sd, B.sort_shadow_bits) : -1);
             }
         } else {
             // Plain passes may bin the next bounce's rays (the record of one bounce carries
             // sort_count) and the deferred shadow rays (origin cells).
             if (B.sort_count) bin_count(B.sort_count, emit_next ? plain_ray_bin(S0, no, nd, B.sort_ray_bits) : -1);
-            if (B.sort_count_shadow) bin_count(B.sort_count_shadow, emit_shadow ? cell_bits(S0, so, DFPT_SHADOW_CELL_BITS) : -1);
+            if (B.sort_count_shadow) bin_count(B.sort_count_shadow, emit_shadow ? cell_bits(S0, so, B.sort_shadow_bits) : -1);
         }
         const int sslot = warp_push(B.counts + DFPT_COUNTS_SHADOW, emit_shadow);
         if (sslot >= 0) {
@@ -1368,7 +1337,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
             if (step)
                 shade_ray<false>(S, Pp, B, Q, b, pass, o, d, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset), path,
                                  emit_next, no, nd, emit_shadow, so, sd, sc);
-            if (B.sort_count_shadow) bin_count(B.sort_count_shadow, emit_shadow ? cell_bits(S, so, DFPT_SHADOW_CELL_BITS) : -1);
+            if (B.sort_count_shadow) bin_count(B.sort_count_shadow, emit_shadow ? cell_bits(S, so, B.sort_shadow_bits) : -1);
             const int sslot = warp_push(B.counts + DFPT_COUNTS_SHADOW, emit_shadow);
             if (sslot >= 0) {
                 B.s_o[sslot] = so;
@@ -1839,7 +1808,7 @@ __global__ void k_bend_wave(DevBatch Q) {
 __global__ void __launch_bounds__(256) k_sort_hist(DevBatch Q, DevPass B, int bounce) {
     const int n = B.counts[bounce + 1];
     const int first = wave_first_scene(Q);
-    GRID_STRIDE_UNIFORM(i, n) bin_count(B.sort_count, i < n ? ray_bin_in_wave(Q, first, B.q_o[1][i], B.q_d[1][i]) : -1);
+    GRID_STRIDE_UNIFORM(i, n) bin_count(B.sort_count, i < n ? ray_bin_in_wave(Q, first, B.q_o[1][i], B.q_d[1][i], B.sort_ray_bits) : -1);
 }
 
 // Moves the shadow queue (B.s_*) into the second set (out) in bin order.
@@ -1853,7 +1822,7 @@ __global__ void __launch_bounds__(256) k_sort_shadow_scatter(DevBatch Q, DevPass
             o = B.s_o[i];
             d = B.s_d[i];
             c = B.s_c[i];
-            key = shadow_bin_in_wave(Q, first, o, d);
+            key = shadow_bin_in_wave(Q, first, o, d, B.sort_shadow_bits);
         }
         const unsigned same = __match_any_sync(0xFFFFFFFFu, key);
         const int leader = __ffs(same) - 1;
@@ -1924,6 +1893,41 @@ __global__ void __launch_bounds__(256) k_sort_chunk_scan(DevPass B, int* counts)
     reinterpret_cast<int4*>(B.sort_bins + (size_t)blockIdx.x * 1024)[threadIdx.x] =
         make_int4(before, before + c.x, before + c.x + c.y, before + c.x + c.y + c.z);
 }
+// The whole scan in one launch of one block, for few bins: 4,096 at a time.
+__global__ void __launch_bounds__(1024) k_sort_scan_small(DevPass B, int* counts, int chunks) {
+    __shared__ int warp_sum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int carry = 0;
+    for (int c0 = 0; c0 < chunks * 256; c0 += 1024) {
+        const int at = c0 + threadIdx.x;  // 4 bins
+        int4* cp = reinterpret_cast<int4*>(counts) + at;
+        int4 c = make_int4(0, 0, 0, 0);
+        if (at < chunks * 256) {
+            c = *cp;
+            *cp = make_int4(0, 0, 0, 0);
+        }
+        const int v = c.x + c.y + c.z + c.w;
+        int x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_sum[w] = x;
+        __syncthreads();
+        int t = warp_sum[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, t, o);
+            if (lane >= o) t += y;
+        }
+        const int total = __shfl_sync(0xFFFFFFFFu, t, 31);
+        const int mine = __shfl_sync(0xFFFFFFFFu, t, w) - warp_sum[w];  // the warps before this one
+        const int before = carry + mine + x - v;
+        if (at < chunks * 256)
+            reinterpret_cast<int4*>(B.sort_bins)[at] = make_int4(before, before + c.x, before + c.x + c.y, before + c.x + c.y + c.z);
+        carry += total;
+        __syncthreads();  // warp_sum is written again
+    }
+}
 // A plain pass's deferred shadow rays into `out` in origin-cell order (the counts come from its
 // shading, the offsets from the scan).
 __global__ void __launch_bounds__(256) k_sort_shadow_scatter_plain(DevScene S, DevPass B, float4* out_o, float4* out_d, float4* out_c) {
@@ -1935,7 +1939,7 @@ __global__ void __launch_bounds__(256) k_sort_shadow_scatter_plain(DevScene S, D
             o = B.s_o[i];
             d = B.s_d[i];
             c = B.s_c[i];
-            key = cell_bits(S, o, DFPT_SHADOW_CELL_BITS);
+            key = cell_bits(S, o, B.sort_shadow_bits);
         }
         const unsigned same = __match_any_sync(0xFFFFFFFFu, key);
         const int leader = __ffs(same) - 1;
@@ -1975,12 +1979,22 @@ __global__ void __launch_bounds__(256) k_sort_rays_scatter_plain(DevScene S, Dev
         }
     }
 }
-// `chunks` chunks of 1024 bins hold every key (keys below chunks x 1024).
-static void launch_sort_scan(const LaunchCtx& c, int* counts, int chunks = DFPT_SORT_CHUNKS) {
+// `chunks` chunks of 1024 bins hold every key (keys below chunks x 1024). Returns the kernels launched.
+static int launch_sort_scan(const LaunchCtx& c, int* counts, long long keys) {
+    const int chunks = (int)((keys + 1023) / 1024);
+    if (chunks <= 32) {  // 8 rounds of one block, less than the three launches
+        k_sort_scan_small<<<1, 1024, 0, c.stream>>>(*c.pass, counts, chunks);
+        return 1;
+    }
     k_sort_chunk_sums<<<chunks, 256, 0, c.stream>>>(*c.pass, counts);
     k_sort_chunk_offsets<<<1, 256, 0, c.stream>>>(*c.pass, chunks);
     k_sort_chunk_scan<<<chunks, 256, 0, c.stream>>>(*c.pass, counts);
+    return 3;
 }
+static long long ray_keys(const LaunchCtx& c, int scenes) {
+    return (scenes > 1 ? 8 * 128ll : (long long)DFPT_RAY_DIRS) << c.pass->sort_ray_bits;
+}
+static long long shadow_keys(const LaunchCtx& c, int scenes) { return (scenes > 1 ? 8ll : 1ll) << c.pass->sort_shadow_bits; }
 
 __global__ void __launch_bounds__(256) k_sort_scatter(DevBatch Q, DevPass B, int bounce) {
     const int n = B.counts[bounce + 1];
@@ -1991,7 +2005,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(DevBatch Q, DevPass B, int
         if (i < n) {
             o = B.q_o[1][i];
             d = B.q_d[1][i];
-            key = ray_bin_in_wave(Q, first, o, d);
+            key = ray_bin_in_wave(Q, first, o, d, B.sort_ray_bits);
         }
         // Lanes with the same bin take consecutive places with one atomic.
         const unsigned same = __match_any_sync(0xFFFFFFFFu, key);
@@ -2307,16 +2321,16 @@ static void launch_b_shadow_reset(const LaunchCtx& c, int) { k_shadow_reset<<<1,
 // Returns the kernels launched.
 static int launch_b_sort(const LaunchCtx& c, int bounce, bool counted) {
     if (!counted) k_sort_hist<<<c.grid, 256, 0, c.stream>>>(*c.batch, *c.pass, bounce);
-    launch_sort_scan(c, c.pass->sort_count);
+    const int k = launch_sort_scan(c, c.pass->sort_count, ray_keys(c, c.batch->n_scenes));
     k_sort_scatter<<<c.grid, 256, 0, c.stream>>>(*c.batch, *c.pass, bounce);
-    return counted ? 4 : 5;
+    return k + (counted ? 1 : 2);
 }
 // Bins the shadow queue into `to` (a pass record whose s_* point at the second set); k_shade
 // counted the bins.
 static int launch_b_sort_shadow(const LaunchCtx& c, const DevPass& to) {
-    launch_sort_scan(c, c.pass->sort_count_shadow);
+    const int k = launch_sort_scan(c, c.pass->sort_count_shadow, shadow_keys(c, c.batch->n_scenes));
     k_sort_shadow_scatter<<<c.grid, 256, 0, c.stream>>>(*c.batch, *c.pass, to.s_o, to.s_d, to.s_c);
-    return 4;
+    return k + 1;
 }
 
 // Path-replay adjoint. Per-primitive partials live in shared memory when they fit in 44 KB.
@@ -2356,20 +2370,18 @@ static void launch_film(const LaunchCtx& c) { k_film<<<c.grid, 256, 0, c.stream>
 static void launch_end_pass(const LaunchCtx& c) { k_end_pass<<<1, 32, 0, c.stream>>>(*c.pass); }
 // Bins a plain pass's deferred shadow rays into `to` (a pass record whose s_* point at the second
 // set); shading counted the bins. Returns the kernels launched.
-static_assert(DFPT_SHADOW_CELL_BITS >= 10 && (1 << DFPT_SHADOW_CELL_BITS) <= DFPT_SORT_BINS,
-              "the plain shadow scan covers whole chunks of 1024 bins within the bin array");
 static int launch_sort_shadow(const LaunchCtx& c, const DevPass& to) {
-    launch_sort_scan(c, c.pass->sort_count_shadow, (1 << DFPT_SHADOW_CELL_BITS) / 1024);
+    const int k = launch_sort_scan(c, c.pass->sort_count_shadow, shadow_keys(c, 1));
     k_sort_shadow_scatter_plain<<<c.grid, 256, 0, c.stream>>>(*c.scene, *c.pass, to.s_o, to.s_d, to.s_c);
-    return 4;
+    return k + 1;
 }
 // Bins the rays a plain pass queued for `bounce` into `to` (a pass record whose queue of that
 // bounce's parity points at the second set); c.pass is the record the shading counted with.
 static int launch_sort_rays(const LaunchCtx& c, int bounce, const DevPass& to) {
     const int qi = bounce & 1;
-    launch_sort_scan(c, c.pass->sort_count, ((96 << c.pass->sort_ray_bits) + 1023) / 1024);
+    const int k = launch_sort_scan(c, c.pass->sort_count, ray_keys(c, 1));
     k_sort_rays_scatter_plain<<<c.grid, 256, 0, c.stream>>>(*c.scene, *c.pass, bounce, to.q_o[qi], to.q_d[qi]);
-    return 4;
+    return k + 1;
 }
 static void launch_film_mean(const LaunchCtx& c, double* out3) { k_film_mean<<<c.grid, 256, 0, c.stream>>>(*c.pass, out3); }
 static void launch_film_average(const LaunchCtx& c, float* rgb, int* samples) {
