@@ -11,9 +11,6 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <future>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "dfpt.h"
@@ -156,6 +153,9 @@ int convert_bvh(const HostScene& s, Derived& d, int root, int& first_node) {
     std::vector<int> index_of_rel(rel + 1, -1);
     for (size_t i = 0; i < offs.size(); ++i) index_of_rel[offs[i]] = (int)i;
     first_node = (int)(d.nodes.size() / 2);
+    const float* P = s.point3fs.data();
+    const int* T = s.triangles.data();
+    bool nested = true;
     for (size_t i = 0; i < offs.size(); ++i) {
         const int at = root + offs[i];
         const int type = s.bvh[at], next = s.bvh[at + 1], mn = s.bvh[at + 2], mx = s.bvh[at + 3];
@@ -167,6 +167,7 @@ int convert_bvh(const HostScene& s, Derived& d, int root, int& first_node) {
         }
         if (!in_range(mn, 3, (int64_t)s.point3fs.size()) || !in_range(mx, 3, (int64_t)s.point3fs.size()))
             return dfpt_fail(DFPT_ERR_INVALID_SCENE, "BVH node at %d has bounds out of range", at);
+        const float lo[3] = {P[mn], P[mn + 1], P[mn + 2]}, hi[3] = {P[mx], P[mx + 1], P[mx + 2]};
         int leaf = -1;
         if (type == 1) {
             if (s.bvh[at + 4] != offs[i] + 5) return dfpt_fail(DFPT_ERR_NOT_SUPPORTED, "BVH node at %d: left child is not the next node", at);
@@ -181,18 +182,24 @@ int convert_bvh(const HostScene& s, Derived& d, int root, int& first_node) {
                     if (r) return r;
                     const int rec = add_tri_record(s, d, toff, k == cnt - 1, first_node + (int)i);
                     if (k == 0) leaf = rec;
+                    for (int v = 0; v < 3; ++v) {
+                        const float* p = P + T[toff + v];
+                        nested &= (p[0] >= lo[0]) & (p[1] >= lo[1]) & (p[2] >= lo[2]) & (p[0] <= hi[0]) & (p[1] <= hi[1]) & (p[2] <= hi[2]);
+                    }
                 }
             }
         }
-        const float* P = s.point3fs.data();
-        d.nodes.push_back(make_float4(P[mn], P[mn + 1], P[mn + 2], int_bits(next_index)));
-        d.nodes.push_back(make_float4(P[mx], P[mx + 1], P[mx + 2], int_bits(leaf)));
+        d.nodes.push_back(make_float4(lo[0], lo[1], lo[2], int_bits(next_index)));
+        d.nodes.push_back(make_float4(hi[0], hi[1], hi[2], int_bits(leaf)));
     }
+    d.nested = d.nested && nested;
     return DFPT_OK;
 }
 
 int build_derived(const HostScene& s, Derived& d) {
     const int np = (int)(s.primitives.size() / 3);
+    d.tris.reserve(s.triangles.size() / 4);  // 3 records per triangle of 12 offsets, and about a node each
+    d.nodes.reserve(s.bvh.size() / 3);
     std::vector<std::pair<int, int>> bvh_roots;  // root offset -> first node
     for (int i = 0; i < np; ++i) {
         const int type = s.primitives[3 * i], off = s.primitives[3 * i + 1], so = s.primitives[3 * i + 2];
@@ -1230,62 +1237,6 @@ int scene_load(const dfpt_scene_desc* sd, SceneStore& st) {
     return DFPT_OK;
 }
 
-// Whether the trees (full and binary, no empty leaf) allow the packed pair walk: every child's box
-// lies in its parent's and every triangle in its leaf's, so a box that the ray enters from outside
-// holds no hit before its entry; finite boxes; at most DFPT_WALK_DEPTH levels below a root. Large
-// trees are checked in parts by up to 8 threads (722 k triangles: 15 ms by one thread, 3 by 8).
-static bool walk_ordered(const HostScene& h, const Derived& d) {
-    const size_t nn = d.nodes.size() / 2;
-    bool any_mesh = false;
-    for (const int4& info : d.prim_info) any_mesh = any_mesh || info.x == DFPT_SHAPE_TRIANGLE_MESH;
-    if (!any_mesh) return false;  // nothing to walk
-    auto inside = [&](size_t n, const float* p) {
-        const float4 lo = d.nodes[2 * n], hi = d.nodes[2 * n + 1];
-        return p[0] >= lo.x && p[0] <= hi.x && p[1] >= lo.y && p[1] <= hi.y && p[2] >= lo.z && p[2] <= hi.z;
-    };
-    auto nested = [&](size_t first, size_t last) {
-        for (size_t n = first; n < last; ++n) {
-            const float4 lo = d.nodes[2 * n], hi = d.nodes[2 * n + 1];
-            if (!(std::isfinite(lo.x) && std::isfinite(lo.y) && std::isfinite(lo.z) && std::isfinite(hi.x) && std::isfinite(hi.y) && std::isfinite(hi.z))) return false;
-            const int leaf = float_bits_int(hi.w);
-            if (leaf == -1) {
-                for (size_t c : {n + 1, (size_t)float_bits_int(d.nodes[2 * (n + 1)].w)}) {
-                    const float4 cl = d.nodes[2 * c], ch = d.nodes[2 * c + 1];
-                    if (!(cl.x <= ch.x && cl.y <= ch.y && cl.z <= ch.z) || !inside(n, &cl.x) || !inside(n, &ch.x)) return false;
-                }
-            } else {
-                for (size_t k = (size_t)leaf;; ++k) {
-                    const int* T = h.triangles.data() + float_bits_int(d.tris[3 * k].w);
-                    for (int v = 0; v < 3; ++v)
-                        if (!inside(n, h.point3fs.data() + T[v])) return false;
-                    if (float_bits_int(d.tris[3 * k + 1].w) != 0) break;
-                }
-            }
-        }
-        return true;
-    };
-    const size_t parts = nn < 16384 ? 1 : std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
-    std::vector<std::future<bool>> others;
-    size_t begun = nn / parts;  // [0, begun) here, the rest by the other threads
-    try {
-        for (size_t p = 1; p < parts; ++p) {
-            const size_t first = nn * p / parts, last = nn * (p + 1) / parts;
-            others.push_back(std::async(std::launch::async, nested, first, last));
-        }
-    } catch (const std::system_error&) {
-        begun = nn;  // no thread to be had: everything here
-    }
-    bool ok = nested(0, begun);
-    std::vector<uint8_t> depth(nn, 0);  // roots at 0; a child comes after its parent in preorder
-    for (size_t n = 0; n < nn && ok; ++n) {
-        if (float_bits_int(d.nodes[2 * n + 1].w) != -1) continue;
-        if (depth[n] >= DFPT_WALK_DEPTH) { ok = false; break; }
-        depth[n + 1] = depth[(size_t)float_bits_int(d.nodes[2 * (n + 1)].w)] = (uint8_t)(depth[n] + 1);
-    }
-    for (auto& f : others) ok = f.get() && ok;
-    return ok;
-}
-
 // Fills the second half of prim_info_host (prim_walk) from the matrices.
 static void fill_walk(SceneStore& st) {
     const float* m = st.host.w2o.data();
@@ -1326,10 +1277,15 @@ int scene_upload(SceneStore& st, cudaStream_t s) {
     fill_walk(st);
     CUDA_TRY(upload(st.prim_info, st.prim_info_host, s));
     {
-        std::vector<float4> trav(d.nodes);
-        trav.insert(trav.end(), d.tris.begin(), d.tris.end());
+        // Nodes and triangles in one allocation (one L2 persistence window).
         st.trav_nodes = d.nodes.size();
-        CUDA_TRY(upload(st.trav, trav, s));
+        const size_t n = d.nodes.size() + d.tris.size();
+        if (!st.trav.p || st.trav.n != n) {
+            st.trav.release();
+            CUDA_TRY(st.trav.alloc(n));
+        }
+        CUDA_TRY(cudaMemcpyAsync(st.trav.p, d.nodes.data(), d.nodes.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
+        CUDA_TRY(cudaMemcpyAsync(st.trav.p + d.nodes.size(), d.tris.data(), d.tris.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
         CUDA_TRY(cudaStreamSynchronize(s));
     }
     {
@@ -1339,22 +1295,36 @@ int scene_upload(SceneStore& st, cudaStream_t s) {
         const size_t nn = d.nodes.size() / 2;
         std::vector<float4> pairs(4 * nn, make_float4(0, 0, 0, 0));
         bool full_binary = true, empty_leaf = false;
+        // The packed pair walk's condition (use_pairs 3): every child's box lies in its parent's (and every
+        // triangle in its leaf's: Derived::nested), so a box that the ray enters from outside holds no hit
+        // before its entry; finite boxes; no tree deeper than the walk's stack.
+        bool nested = d.nested;
+        std::vector<uint8_t> depth(nn, 0);  // roots at 0; a child comes after its parent in preorder
         auto next_of = [&](size_t n) { return float_bits_int(d.nodes[2 * n].w); };
         auto leaf_of = [&](size_t n) { return float_bits_int(d.nodes[2 * n + 1].w); };
         for (size_t n = 0; n < nn && full_binary; ++n) {
+            const float4 nl = d.nodes[2 * n], nh = d.nodes[2 * n + 1];
+            nested = nested && std::isfinite(nl.x) && std::isfinite(nl.y) && std::isfinite(nl.z) && std::isfinite(nh.x) &&
+                     std::isfinite(nh.y) && std::isfinite(nh.z);
             if (leaf_of(n) == -2) empty_leaf = true;
             if (leaf_of(n) != -1) continue;
             const size_t l = n + 1;
             const int r = l < nn ? next_of(l) : -1;
             if (l >= nn || r < 0 || (size_t)r >= nn || next_of((size_t)r) != next_of(n)) { full_binary = false; break; }
             const float4 lo = d.nodes[2 * l], lh = d.nodes[2 * l + 1], ro = d.nodes[2 * (size_t)r], rh = d.nodes[2 * (size_t)r + 1];
+            auto inside = [&](const float4& cl, const float4& ch) {
+                return cl.x >= nl.x && cl.y >= nl.y && cl.z >= nl.z && ch.x <= nh.x && ch.y <= nh.y && ch.z <= nh.z && cl.x <= ch.x &&
+                       cl.y <= ch.y && cl.z <= ch.z;
+            };
+            nested = nested && depth[n] < DFPT_WALK_DEPTH && inside(lo, lh) && inside(ro, rh);
+            depth[l] = depth[(size_t)r] = (uint8_t)std::min(depth[n] + 1, DFPT_WALK_DEPTH);
             auto code = [&](int leaf, int node) { return leaf == -1 ? node : leaf == -2 ? INT32_MIN : ~leaf; };
             pairs[4 * n] = make_float4(lo.x, lo.y, lh.x, lh.y);
             pairs[4 * n + 1] = make_float4(ro.x, ro.y, rh.x, rh.y);
             pairs[4 * n + 2] = make_float4(lo.z, lh.z, ro.z, rh.z);
             pairs[4 * n + 3] = make_float4(int_bits(code(leaf_of(l), (int)l)), int_bits(code(leaf_of((size_t)r), r)), int_bits(r), 0.0f);
         }
-        st.scene.use_pairs = !full_binary ? 0 : empty_leaf ? 1 : walk_ordered(h, d) ? 3 : 2;
+        st.scene.use_pairs = !full_binary ? 0 : empty_leaf ? 1 : nested ? 3 : 2;
         st.scene.pair_stack = 8;
         CUDA_TRY(upload(st.pairs, pairs, s));
         CUDA_TRY(cudaStreamSynchronize(s));
