@@ -611,9 +611,9 @@ void fill_dev_params(dfpt_handle* h) {
     // Tile slot order: the counter stream keys samples by pixel, so the order is free; the LCG's
     // per-pixel states, the wireframe overlay's per-pixel rays and the adjoint's per-pixel records
     // keep slot = pixel.
-    // The per-pixel modes (k_simple) write their results at slot = pixel.
+    // The per-pixel modes (k_simple) take pixels in the same order but keep their results at slot = pixel.
     d.pixel_tiles = (h->pixel_tiles && h->params.rng_kind == DFPT_RNG_COUNTER && h->params.wireframes != 1 && !h->diff_on &&
-                     !is_simple_mode(h->params.renderer_type) && h->width % 8 == 0 && h->height % 4 == 0) ? 1 : 0;
+                     !is_simple_mode(h->params.renderer_type)) ? 1 : 0;
     if (h->diff_on) {
         d.diff = 1;
         d.diff_pass0 = h->diff_pass0;

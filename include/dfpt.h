@@ -238,8 +238,8 @@ int dfpt_read_profile(dfpt_handle* handle, double* ms_by_kind10, int32_t* launch
  *   "wide_samples"      passes per wave when dfpt_render renders several passes (1..64, default
  *                       8; 1 renders pass by pass); the film is the same either way;
  *   "pixel_tiles"       1 (default) runs a plain pass's queue slots over 8 x 4 pixel tiles (a warp's
- *                       primary rays leave a compact block of pixels; width a multiple of 8, height
- *                       of 4, counter-based RNG, path tracer without wireframes), 0 in row order;
+ *                       primary rays leave a compact block of pixels; counter-based RNG, path tracer
+ *                       without wireframes), 0 in row order;
  *   "tail_bounce"       t >= 0: a plain pass runs bounces t .. depth-1 and the final any-hit of each
  *                       path in one launch (same steps per path; t = 0 includes the camera rays'
  *                       traversal and shading); -1 (default) a launch per bounce;
