@@ -110,9 +110,11 @@ def _scene(name):
     if name == "sphere":
         pos, idx, _, _, _ = synthetic.displaced_icosphere(6, 0.2, 4, radius=1.7)
         return _mesh_scene(pos, idx)
-    if name in ("shared_matrix", "own_matrices", "many"):
-        pos, idx, _, _, _ = synthetic.displaced_icosphere(3, 0.2, 4, radius=0.9)
-        return _mesh_scene(pos, idx, copies=12 if name == "many" else 4, spread=0.0 if name == "shared_matrix" else 1.8)
+    if name in ("shared_matrix", "own_matrices", "many", "crowd"):
+        # A ray through the crowd enters up to 70 boxes, more than a round of 16 candidates.
+        pos, idx, _, _, _ = synthetic.displaced_icosphere(3, 0.2, 4, radius=0.9 if name != "crowd" else 0.3)
+        copies, spread = {"shared_matrix": (4, 0.0), "own_matrices": (4, 1.8), "many": (12, 1.8), "crowd": (70, 0.9)}[name]
+        return _mesh_scene(pos, idx, copies=copies, spread=spread)
     count = {"one": 1, "two": 2, "five": 5, "chain": 40, "deepest": 65, "too_deep": 66, "not_nested": 9}[name]
     compiled, sky, params = _mesh_scene(*_triangles(count))
     if name in ("chain", "deepest", "too_deep"):
@@ -141,7 +143,7 @@ def _render(compiled, sky, params, counting, culling, passes):
     return out
 
 
-@pytest.mark.parametrize("name", ["one", "two", "five", "sphere", "chain", "deepest", "too_deep", "not_nested", "shared_matrix", "own_matrices", "many",
+@pytest.mark.parametrize("name", ["one", "two", "five", "sphere", "chain", "deepest", "too_deep", "not_nested", "shared_matrix", "own_matrices", "many", "crowd",
                                   "flat_sphere_0", "flat_sphere_3", "flat_sphere_8", "flat_sphere_90", "flat_sphere_90_twice", "flat_triangle_30",
                                   "flat_triangle_30_twice"])
 def test_packed_walk_equals_counting_walk(name):
