@@ -626,15 +626,38 @@ __device__ __forceinline__ unsigned wave_passes(const DevBatch& Q, long long np)
     const long long end = base + Q.capacity < Q.wave_base[1] ? base + Q.capacity : Q.wave_base[1];
     return (unsigned)((end - base) / np);
 }
-__device__ __forceinline__ unsigned slot_of_rel(unsigned rel, unsigned np, unsigned passes) {
-    if (passes == 0u) return rel;
-    const unsigned j = rel / np;
-    return (rel - j * np) * passes + j;
+#endif
+// What a kernel derives from the wave once per thread, before its loop: the slots' pixels and passes
+// follow with one division each by a small number (the wave's passes) instead of 64-bit ones.
+struct WavePixels {
+    unsigned np;        // pixels
+    unsigned passes;    // passes of the wave (pixel-major slots), or 0 in sample order
+    unsigned inverse;   // 2^32 / passes rounded up
+    long long base;     // the wave's first sample
+    long long first;    // its pass in the render (with passes)
+    uint32_t rng_pass;  // its RNG pass (with passes)
+};
+#ifdef DFPT_ONE_SCENE
+__device__ __forceinline__ WavePixels wave_pixels(const DevBatch& Q) {
+    WavePixels w;
+    w.np = (unsigned)((long long)Q.params[0].width * Q.params[0].height);
+    w.passes = wave_passes(Q, w.np);
+    w.inverse = w.passes > 1u ? 0xFFFFFFFFu / w.passes + 1u : 0u;
+    w.base = Q.wave_base[0];
+    w.first = w.passes ? w.base / w.np : 0;
+    w.rng_pass = (uint32_t)(w.first + Q.wave_base[2]);
+    return w;
 }
-__device__ __forceinline__ unsigned rel_of_slot(unsigned slot, unsigned np, unsigned passes) {
-    if (passes == 0u) return slot;
-    const unsigned x = slot / passes;
-    return (slot - x * passes) * np + x;
+// Slot -> pixel and place among the pixel's passes, pixel-major (at most one too high before the check:
+// slots stay below 2^27 and passes at most 64).
+__device__ __forceinline__ void pixel_of_wave_slot(const WavePixels& w, unsigned slot, unsigned& pixel, unsigned& j) {
+    pixel = w.passes > 1u ? __umulhi(slot, w.inverse) : slot;
+    int r = (int)(slot - pixel * w.passes);
+    if (r < 0) {
+        --pixel;
+        r += (int)w.passes;
+    }
+    j = (unsigned)r;
 }
 #endif
 
@@ -684,7 +707,7 @@ __global__ void __launch_bounds__(256) k_camera(DevScene S0, const DevParams* __
         pass0 = Q.wave_base[2];
     }
 #ifdef DFPT_ONE_SCENE
-    const unsigned wave_p = wave_passes(Q, (long long)Q.params[0].width * Q.params[0].height);
+    const WavePixels wave = wave_pixels(Q);
 #endif
     // A thin lens keeps every pixel, so with one scene the queue is the slots in order (no atomics):
     // the valid slots are a prefix.
@@ -701,14 +724,22 @@ __global__ void __launch_bounds__(256) k_camera(DevScene S0, const DevParams* __
         if constexpr (BATCH) {
             if (valid) {
 #ifdef DFPT_ONE_SCENE
-                // Slots past the wave's samples stay invalid (rel_of_slot maps only those below).
-                const unsigned np0 = (unsigned)((long long)Q.params[0].width * Q.params[0].height);
-                const long long g = wave_p == 0u ? base + i
-                                    : (unsigned)i < wave_p * np0 ? base + rel_of_slot((unsigned)i, np0, wave_p) : end;
+                // Slots past the wave's samples stay invalid.
+                const bool by_pixel = wave.passes != 0u;
+                if (by_pixel) {
+                    unsigned x, j;
+                    pixel_of_wave_slot(wave, (unsigned)i, x, j);
+                    pixel = (int)x;
+                    sample = wave.rng_pass + j;
+                    valid = x < wave.np;
+                    if (valid && Q.params[0].diff) Q.slot_key[i] = make_int4(0, pixel, (int)sample, 0);  // the adjoint replay reads it
+                }
 #else
-                const long long g = base + i;
+                const bool by_pixel = false;
 #endif
-                if (g >= end) {
+                const long long g = base + i;
+                if (by_pixel) {
+                } else if (g >= end) {
                     valid = false;
                 } else {
                     sid = batch_scene_of(Q, g);
@@ -1019,8 +1050,8 @@ __device__ __forceinline__ void bin_count(int* bins, int key) {
 // place. Returns the next ray in (emit_next, no, nd) and the sun shadow ray in (emit_shadow, so,
 // sd, sc); the caller queues them.
 template <bool BATCH>
-__device__ __forceinline__ void shade_ray(const DevScene& S0, const DevParams* __restrict__ Pp, DevPass& B, const DevBatch& Q, int bounce,
-                                          uint32_t pass, const float4 o4, const float4 d4, const int4 hr, int& path, bool& emit_next,
+__device__ __forceinline__ void shade_ray(const DevScene& S0, const DevParams* __restrict__ Pp, DevPass& B, const DevBatch& Q, const WavePixels& wave,
+                                          int bounce, uint32_t pass, const float4 o4, const float4 d4, const int4 hr, int& path, bool& emit_next,
                                           float4& no, float4& nd, bool& emit_shadow, float4& so, float4& sd, float4& sc) {
     path = __float_as_int(o4.w);
     const int sid = BATCH ? __float_as_int(d4.w) : 0;
@@ -1030,17 +1061,15 @@ __device__ __forceinline__ void shade_ray(const DevScene& S0, const DevParams* _
     uint32_t rng_pixel = (uint32_t)(BATCH ? path : pixel_of_slot(P, path)), rng_pass = pass;
     if constexpr (BATCH) {
 #ifdef DFPT_ONE_SCENE
-        // One scene: the slot's pixel and pass follow from its index as k_camera derived
-        // them (slot i of the wave is sample base + i), without the random slot-key load.
-        const long long np = (long long)P.width * P.height;
-        const long long local = Q.wave_base[0] + rel_of_slot((unsigned)path, (unsigned)np, wave_passes(Q, np)) - Q.sample_begin[0];
-        if (local < 0x7FFFFFFFll) {
-            const unsigned q = (unsigned)local / (unsigned)np;
-            rng_pixel = (unsigned)local - q * (unsigned)np;
-            rng_pass = (uint32_t)(q + Q.wave_base[2]);
+        // One scene: the slot's pixel and pass follow from its index as k_camera derived them (slot i of
+        // the wave is sample base + i), without the random slot-key load.
+        if (wave.passes != 0u) {
+            unsigned j;
+            pixel_of_wave_slot(wave, (unsigned)path, rng_pixel, j);
+            rng_pass = wave.rng_pass + j;
         } else {
-            const long long j = local / np;
-            rng_pixel = (uint32_t)(local - j * np);
+            const long long local = wave.base + path, j = local / wave.np;
+            rng_pixel = (uint32_t)(local - j * wave.np);
             rng_pass = (uint32_t)(j + Q.wave_base[2]);
         }
 #else
@@ -1144,12 +1173,17 @@ __global__ void __launch_bounds__(256, DFPT_SHADE_MINB) k_shade(DevScene S0, con
     const int n = B.counts[bounce];
     const int qi = B.sorted_queues ? 0 : (bounce & 1);
     const uint32_t pass = BATCH ? 0u : (uint32_t)*B.pass_index;
+#ifdef DFPT_ONE_SCENE
+    const WavePixels wave = wave_pixels(Q);
+#else
+    const WavePixels wave{};
+#endif
     GRID_STRIDE_UNIFORM(i, n) {
         bool emit_next = false, emit_shadow = false;
         float4 no = make_float4(0, 0, 0, 0), nd = make_float4(0, 0, 0, 0);
         float4 so = make_float4(0, 0, 0, 0), sd = make_float4(0, 0, 0, 0), sc = make_float4(0, 0, 0, 0);
         int path = 0;
-        if (i < n) shade_ray<BATCH>(S0, Pp, B, Q, bounce, pass, B.q_o[qi][i], B.q_d[qi][i], B.q_hit[i], path, emit_next, no, nd,
+        if (i < n) shade_ray<BATCH>(S0, Pp, B, Q, wave, bounce, pass, B.q_o[qi][i], B.q_d[qi][i], B.q_hit[i], path, emit_next, no, nd,
                                     emit_shadow, so, sd, sc);
         const int slot = warp_push(B.counts + bounce + 1, emit_next);
         if (slot >= 0) {
@@ -1343,7 +1377,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
             float4 so = make_float4(0, 0, 0, 0), sd = make_float4(0, 0, 0, 0), sc = make_float4(0, 0, 0, 0);
             int path = 0;
             if (step)
-                shade_ray<false>(S, Pp, B, Q, b, pass, o, d, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset), path,
+                shade_ray<false>(S, Pp, B, Q, WavePixels{}, b, pass, o, d, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset), path,
                                  emit_next, no, nd, emit_shadow, so, sd, sc);
             if (B.sort_count_shadow) bin_count(B.sort_count_shadow, emit_shadow ? cell_bits(S, so, B.sort_shadow_bits) : -1);
             const int sslot = warp_push(B.counts + DFPT_COUNTS_SHADOW, emit_shadow);
@@ -1752,6 +1786,9 @@ __global__ void __launch_bounds__(256) k_bfilm(DevBatch Q, DevPass B) {
     const long long tasks = Q.wave_tab[4 * E + 3];
     const long long base = Q.wave_base[0];
     const long long clear_sample = Q.wave_base[3];
+#ifdef DFPT_ONE_SCENE
+    const WavePixels wave = wave_pixels(Q);
+#endif
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tasks; t += (long long)gridDim.x * blockDim.x) {
         int e = 0;
         while (e + 1 < E && Q.wave_tab[4 * (e + 1) + 3] <= t) ++e;
@@ -1767,11 +1804,20 @@ __global__ void __launch_bounds__(256) k_bfilm(DevBatch Q, DevPass B) {
         const DevParams& P = Q.params[s];
         const long long pass0 = Q.wave_base[2];
 #ifdef DFPT_ONE_SCENE
-        const unsigned wave_p = wave_passes(Q, np);
+        if (wave.passes != 0u && !P.diff) {
+            // Whole passes of one scene: the pixel's samples lie side by side, in pass order.
+            for (unsigned j = 0; j < wave.passes; ++j) {
+                const size_t slot = (size_t)pixel * wave.passes + j;
+                film_add(B.radiance[PSI(slot)], B.pixel_flags[slot], wave.first + j == clear_sample, sum, comp, cnt);
+            }
+            B.film_sum[f] = sum; B.film_comp[f] = comp; B.film_n[f] = cnt;
+            continue;
+        }
 #endif
         for (long long loc = first; loc < b; loc += np) {
 #ifdef DFPT_ONE_SCENE
-            const int slot = (int)slot_of_rel((unsigned)(slot0 + loc), (unsigned)np, wave_p);
+            const long long rel = slot0 + loc;  // the sample's place in the wave
+            const int slot = (int)(wave.passes == 0u ? rel : (rel % np) * wave.passes + rel / np);
 #else
             const int slot = (int)(slot0 + a + seg_pos_of_local(loc, a, b, np));
 #endif
