@@ -2143,6 +2143,21 @@ __global__ void k_init_tables(const int* perm256, const float* grad36) {
 // Resident blocks of 256 for scenes without meshes: 4 (48-56 registers, no spills); 5, 6 and 8 measured
 // 0.46, 0.50 and 0.76 ms against 0.44 for the closest hits of 64 passes of sphere_scene.
 #define DFPT_FLAT_MINB 4
+// A grid of every block of a kernel that the device holds at once, found once per process. Camera and film
+// ran on k_shade's grid, 3 blocks of 256 per SM, where 5 and 8 fit: 8 frames at 1080p 0.34 -> 0.31 and 0.60
+// -> 0.41 ms. The binning's scatters stay on that grid: with 8 blocks 3.58 -> 3.82 ms of a 32-pass still,
+// their writes spread over more bins at a time.
+template <auto Kernel>
+static int full_grid(int block) {
+    static const int grid = [](int block) {
+        int dev = 0, sms = 0, b = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, Kernel, block, 0);
+        return (sms > 0 ? sms : 1) * (b > 0 ? b : 1);
+    }(block);
+    return grid;
+}
 // A grid of every block of `kernel` that the current device holds at once.
 template <class Kernel>
 static int resident_grid(Kernel kernel, int block, size_t dynamic_shared = 0) {
@@ -2345,7 +2360,7 @@ static int trace_grid(int config, int sms) {
 }
 
 #ifndef DFPT_ONE_SCENE
-static void launch_camera(const LaunchCtx& c) { k_camera<false><<<c.grid, 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}); }
+static void launch_camera(const LaunchCtx& c) { k_camera<false><<<full_grid<k_camera<false>>(256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}); }
 static void launch_shade(const LaunchCtx& c, int bounce) { k_shade<false><<<c.grid, 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce); }
 #endif
 
@@ -2367,11 +2382,11 @@ BATCH_DISPATCH(final)
 #undef BATCH_CASE_closest
 #undef BATCH_CASE_shadow
 #undef BATCH_CASE_final
-static void launch_b_camera(const LaunchCtx& c, int) { k_camera<true><<<c.grid, 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch); }
+static void launch_b_camera(const LaunchCtx& c, int) { k_camera<true><<<full_grid<k_camera<true>>(256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch); }
 static void launch_b_shade(const LaunchCtx& c, int bounce) { k_shade<true><<<c.grid, 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce); }
 static void launch_b_wave(const LaunchCtx& c, int) { k_bwave<<<1, 32, 0, c.stream>>>(*c.batch); }
-static void launch_b_film(const LaunchCtx& c, int) { k_bfilm<<<c.grid, 256, 0, c.stream>>>(*c.batch, *c.pass); }
-static void launch_b_resolve(const LaunchCtx& c, int) { k_bresolve<<<c.grid, 256, 0, c.stream>>>(*c.batch, *c.pass); }
+static void launch_b_film(const LaunchCtx& c, int) { k_bfilm<<<full_grid<k_bfilm>(256), 256, 0, c.stream>>>(*c.batch, *c.pass); }
+static void launch_b_resolve(const LaunchCtx& c, int) { k_bresolve<<<full_grid<k_bresolve>(256), 256, 0, c.stream>>>(*c.batch, *c.pass); }
 static void launch_b_end(const LaunchCtx& c, int) { k_bend_wave<<<1, 32, 0, c.stream>>>(*c.batch); }
 static void launch_b_shadow_reset(const LaunchCtx& c, int) { k_shadow_reset<<<1, 32, 0, c.stream>>>(*c.pass); }
 // Bins the rays shading queued for bounce + 1 (queue 1 -> queue 0). k_shade counts the bins as it
@@ -2424,7 +2439,7 @@ static void launch_simple(const LaunchCtx& c) {
     else k_simple<0><<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
 }
 static void launch_wireframe(const LaunchCtx& c) { k_wireframe<<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass); }
-static void launch_film(const LaunchCtx& c) { k_film<<<c.grid, 256, 0, c.stream>>>(c.params, *c.pass); }
+static void launch_film(const LaunchCtx& c) { k_film<<<full_grid<k_film>(256), 256, 0, c.stream>>>(c.params, *c.pass); }
 static void launch_end_pass(const LaunchCtx& c) { k_end_pass<<<1, 32, 0, c.stream>>>(*c.pass); }
 // Bins a plain pass's deferred shadow rays into `to` (a pass record whose s_* point at the second
 // set); shading counted the bins. Returns the kernels launched.
@@ -2441,9 +2456,9 @@ static int launch_sort_rays(const LaunchCtx& c, int bounce, const DevPass& to) {
     k_sort_rays_scatter_plain<<<c.grid, 256, 0, c.stream>>>(*c.scene, *c.pass, bounce, to.q_o[qi], to.q_d[qi]);
     return k + 1;
 }
-static void launch_film_mean(const LaunchCtx& c, double* out3) { k_film_mean<<<c.grid, 256, 0, c.stream>>>(*c.pass, out3); }
+static void launch_film_mean(const LaunchCtx& c, double* out3) { k_film_mean<<<full_grid<k_film_mean>(256), 256, 0, c.stream>>>(*c.pass, out3); }
 static void launch_film_average(const LaunchCtx& c, float* rgb, int* samples) {
-    k_film_average<<<c.grid, 256, 0, c.stream>>>(*c.pass, rgb, samples);
+    k_film_average<<<full_grid<k_film_average>(256), 256, 0, c.stream>>>(*c.pass, rgb, samples);
 }
 #endif
 static void launch_init_tables(cudaStream_t s, const int* perm, const float* grad) { k_init_tables<<<1, 512, 0, s>>>(perm, grad); }
