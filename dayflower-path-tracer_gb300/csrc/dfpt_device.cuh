@@ -827,6 +827,9 @@ template <bool ANY, int NT>
 __device__ __forceinline__ bool pair_walk(const DevScene& S, int root, float ox, float oy, float oz, float dx, float dy, float dz,
                                           const SlabRay2& sr, float& closest, int& best) {
     constexpr int DONE = (int)0x80000000;  // no triangle's complement
+    // In a batch S lies in global memory: its pointers are read once, not behind every store to the stack.
+    const float4* const pairs = S.pairs;
+    const float4* const tris = S.tris;
     int2* const stk = walk_stack<NT>();
     int2 deep[DFPT_WALK_DEPTH - DFPT_WALK_STACK];
     int top = 0;
@@ -856,7 +859,7 @@ __device__ __forceinline__ bool pair_walk(const DevScene& S, int root, float ox,
     while (code != DONE) {
         while (code >= 0) {
             float4 a, b, c, e;
-            const float4* P = S.pairs + 4 * (size_t)code;
+            const float4* P = pairs + 4 * (size_t)code;
             ldg256(P, a, b);
             ldg256(P + 2, c, e);
             float lmin, lmax, rmin, rmax;
@@ -879,9 +882,9 @@ __device__ __forceinline__ bool pair_walk(const DevScene& S, int root, float ox,
         }
         if (code == DONE) break;
         for (int k = ~code;; ++k) {
-            const float4 a = __ldg(S.tris + 3 * k);
-            const float4 e0 = __ldg(S.tris + 3 * k + 1);
-            const float4 e1 = __ldg(S.tris + 3 * k + 2);
+            const float4 a = __ldg(tris + 3 * k);
+            const float4 e0 = __ldg(tris + 3 * k + 1);
+            const float4 e1 = __ldg(tris + 3 * k + 2);
             const float t = isect_triangle(ox, oy, oz, dx, dy, dz, a, e0, e1, INF);
             if constexpr (ANY) {
                 if (t < INF) {
