@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
             float4 T = B.throughput[PSI(path)];
             float4 Lu = B.radiance[PSI(path)];  // radiance gathered so far along the replay
             const float4 Lt = B.diff_L[sample * npix + pixel];
-            float4 w = B.diff_dldi[pixel];
-            w.x *= inv_spp; w.y *= inv_spp; w.z *= inv_spp;
+            const float* dl = B.diff_dldi + 3 * (size_t)pixel;
+            const float3 w = make_float3(dl[0] * inv_spp, dl[1] * inv_spp, dl[2] * inv_spp);
             if (h.t == INF || h.prim == -1) {
                 D4 sr, sg, sb;
                 sky_color_tan(P, d4.x, d4.y, d4.z, sr, sg, sb);
@@ -432,8 +432,8 @@ __global__ void __launch_bounds__(256) k_final_adj(DevScene S, const DevParams* 
             const float4 T = B.throughput[PSI(path)];
             int pixel = path;
             if constexpr (BATCH) pixel = Q.slot_key[path].y;
-            float4 w = B.diff_dldi[pixel];
-            w.x *= inv_spp; w.y *= inv_spp; w.z *= inv_spp;
+            const float* dl = B.diff_dldi + 3 * (size_t)pixel;
+            const float3 w = make_float3(dl[0] * inv_spp, dl[1] * inv_spp, dl[2] * inv_spp);
             D4 sr, sg, sb;
             sky_color_tan(P, d.x, d.y, d.z, sr, sg, sb);
             for (int j = 0; j < 4; ++j) gsky[j] += (w.x * T.x * sr.d[j] + w.y * T.y * sg.d[j] + w.z * T.z * sb.d[j]) * INV_PI;

@@ -431,8 +431,8 @@ struct dfpt_handle {
     bool diff_ready = false;  // the last forward's samples are stored for a backward
     int diff_pass0 = 0, diff_spp = 0;
     size_t diff_capacity = 0;  // samples x pixels the per-sample records hold
-    DevBuf<float4> diff_albedo, diff_emission, diff_L, diff_dldi;
-    DevBuf<float> diff_exponent, diff_sky_tan;
+    DevBuf<float4> diff_albedo, diff_emission, diff_L;
+    DevBuf<float> diff_exponent, diff_sky_tan, diff_dldi;
     DevBuf<int> vis, diff_vis;
     DevBuf<double> diff_rows, diff_out;
     // Graph of one pass.
@@ -2065,7 +2065,7 @@ int dfpt_diff_forward(dfpt_handle* h, const dfpt_diff_params* dp, int32_t spp, f
         CUDA_TRY(h->diff_vis.alloc((size_t)spp * n));
         h->diff_capacity = (size_t)spp * n;
     }
-    if (!h->diff_dldi.p) CUDA_TRY(h->diff_dldi.alloc(n));
+    if (!h->diff_dldi.p) CUDA_TRY(h->diff_dldi.alloc(3 * n));
     const int rows = std::max(h->ctx.grid, 1), row_len = np * DFPT_DIFF_PER_PRIM + DFPT_DIFF_GLOBAL;
     if (h->diff_rows.n != (size_t)rows * row_len) {
         h->diff_rows.release();
@@ -2098,9 +2098,8 @@ int dfpt_diff_backward(dfpt_handle* h, const float* dloss_dimage, double* grad_a
     const int np = h->sc.scene.primitive_count;
     const int row_len = np * DFPT_DIFF_PER_PRIM + DFPT_DIFF_GLOBAL;
     const int rows = (int)(h->diff_rows.n / (size_t)row_len);
-    std::vector<float4> w(n);
-    for (size_t i = 0; i < n; ++i) w[i] = make_float4(dloss_dimage[3 * i], dloss_dimage[3 * i + 1], dloss_dimage[3 * i + 2], 0.0f);
-    CUDA_TRY(upload(h->diff_dldi, w, h->stream));
+    // As the caller laid it out (4 MB of float4 records built here first took 0.4 ms of 4.0 at 512 x 512).
+    CUDA_TRY(cudaMemcpyAsync(h->diff_dldi.p, dloss_dimage, 3 * n * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(cudaMemsetAsync(h->diff_rows.p, 0, h->diff_rows.n * sizeof(double), h->stream));
     refresh_walk(h);
     // Replay the forward's passes: same pass indices, so the same RNG streams.
@@ -2108,7 +2107,10 @@ int dfpt_diff_backward(dfpt_handle* h, const float* dloss_dimage, double* grad_a
     if (h->diff_spp >= 2 && wide_eligible(h) && h->wide.b_shade_adj) {
         // In waves of wide_samples passes through the batch stages (slot keys give pixel and pass).
         int r = wide_prepare(h);
-        if (r) return r;
+        if (r) {
+            (void)cudaStreamSynchronize(h->stream);  // the copy above reads the caller's memory
+            return r;
+        }
         h->wide_range[0] = 0;
         h->wide_range[1] = (long long)h->diff_spp * h->n_pixels;
         h->wide_range[2] = pass0;

@@ -157,7 +157,7 @@ struct DevPass {
     int* vis;                  // per path: bit b = the sun shadow ray of bounce b was unoccluded
     float4* diff_L;            // [sample][pixel] path radiance of the forward's samples
     int* diff_vis;             // [sample][pixel] the forward's visibility bits
-    const float4* diff_dldi;   // per pixel dLoss/dImage (rgb)
+    const float* diff_dldi;    // 3 per pixel: dLoss/dImage (rgb), as the caller passed it
     double* diff_rows;         // per block of the adjoint kernels: gradient partials
     int diff_row_len;          // primitives x 7 + 4
     // Ray binning between bounces (wide passes): with sorted_queues set, shading writes queue 1,
