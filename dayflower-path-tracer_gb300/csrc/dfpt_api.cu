@@ -154,8 +154,6 @@ int convert_bvh(const HostScene& s, Derived& d, int root, int& first_node) {
     for (size_t i = 0; i < offs.size(); ++i) index_of_rel[offs[i]] = (int)i;
     first_node = (int)(d.nodes.size() / 2);
     const float* P = s.point3fs.data();
-    const int* T = s.triangles.data();
-    bool nested = true;
     for (size_t i = 0; i < offs.size(); ++i) {
         const int at = root + offs[i];
         const int type = s.bvh[at], next = s.bvh[at + 1], mn = s.bvh[at + 2], mx = s.bvh[at + 3];
@@ -167,7 +165,6 @@ int convert_bvh(const HostScene& s, Derived& d, int root, int& first_node) {
         }
         if (!in_range(mn, 3, (int64_t)s.point3fs.size()) || !in_range(mx, 3, (int64_t)s.point3fs.size()))
             return dfpt_fail(DFPT_ERR_INVALID_SCENE, "BVH node at %d has bounds out of range", at);
-        const float lo[3] = {P[mn], P[mn + 1], P[mn + 2]}, hi[3] = {P[mx], P[mx + 1], P[mx + 2]};
         int leaf = -1;
         if (type == 1) {
             if (s.bvh[at + 4] != offs[i] + 5) return dfpt_fail(DFPT_ERR_NOT_SUPPORTED, "BVH node at %d: left child is not the next node", at);
@@ -182,17 +179,12 @@ int convert_bvh(const HostScene& s, Derived& d, int root, int& first_node) {
                     if (r) return r;
                     const int rec = add_tri_record(s, d, toff, k == cnt - 1, first_node + (int)i);
                     if (k == 0) leaf = rec;
-                    for (int v = 0; v < 3; ++v) {
-                        const float* p = P + T[toff + v];
-                        nested &= (p[0] >= lo[0]) & (p[1] >= lo[1]) & (p[2] >= lo[2]) & (p[0] <= hi[0]) & (p[1] <= hi[1]) & (p[2] <= hi[2]);
-                    }
                 }
             }
         }
-        d.nodes.push_back(make_float4(lo[0], lo[1], lo[2], int_bits(next_index)));
-        d.nodes.push_back(make_float4(hi[0], hi[1], hi[2], int_bits(leaf)));
+        d.nodes.push_back(make_float4(P[mn], P[mn + 1], P[mn + 2], int_bits(next_index)));
+        d.nodes.push_back(make_float4(P[mx], P[mx + 1], P[mx + 2], int_bits(leaf)));
     }
-    d.nested = d.nested && nested;
     return DFPT_OK;
 }
 
@@ -1295,28 +1287,18 @@ int scene_upload(SceneStore& st, cudaStream_t s) {
         const size_t nn = d.nodes.size() / 2;
         std::vector<float4> pairs(4 * nn, make_float4(0, 0, 0, 0));
         bool full_binary = true, empty_leaf = false;
-        // The packed pair walk's condition (use_pairs 3): every child's box lies in its parent's (and every
-        // triangle in its leaf's: Derived::nested), so a box that the ray enters from outside holds no hit
-        // before its entry; finite boxes; no tree deeper than the walk's stack.
-        bool nested = d.nested;
+        bool deep = false;  // a tree deeper than the packed pair walk's stack
         std::vector<uint8_t> depth(nn, 0);  // roots at 0; a child comes after its parent in preorder
         auto next_of = [&](size_t n) { return float_bits_int(d.nodes[2 * n].w); };
         auto leaf_of = [&](size_t n) { return float_bits_int(d.nodes[2 * n + 1].w); };
         for (size_t n = 0; n < nn && full_binary; ++n) {
-            const float4 nl = d.nodes[2 * n], nh = d.nodes[2 * n + 1];
-            nested = nested && std::isfinite(nl.x) && std::isfinite(nl.y) && std::isfinite(nl.z) && std::isfinite(nh.x) &&
-                     std::isfinite(nh.y) && std::isfinite(nh.z);
             if (leaf_of(n) == -2) empty_leaf = true;
             if (leaf_of(n) != -1) continue;
             const size_t l = n + 1;
             const int r = l < nn ? next_of(l) : -1;
             if (l >= nn || r < 0 || (size_t)r >= nn || next_of((size_t)r) != next_of(n)) { full_binary = false; break; }
             const float4 lo = d.nodes[2 * l], lh = d.nodes[2 * l + 1], ro = d.nodes[2 * (size_t)r], rh = d.nodes[2 * (size_t)r + 1];
-            auto inside = [&](const float4& cl, const float4& ch) {
-                return cl.x >= nl.x && cl.y >= nl.y && cl.z >= nl.z && ch.x <= nh.x && ch.y <= nh.y && ch.z <= nh.z && cl.x <= ch.x &&
-                       cl.y <= ch.y && cl.z <= ch.z;
-            };
-            nested = nested && depth[n] < DFPT_WALK_DEPTH && inside(lo, lh) && inside(ro, rh);
+            deep = deep || depth[n] >= DFPT_WALK_DEPTH;
             depth[l] = depth[(size_t)r] = (uint8_t)std::min(depth[n] + 1, DFPT_WALK_DEPTH);
             auto code = [&](int leaf, int node) { return leaf == -1 ? node : leaf == -2 ? INT32_MIN : ~leaf; };
             pairs[4 * n] = make_float4(lo.x, lo.y, lh.x, lh.y);
@@ -1324,7 +1306,7 @@ int scene_upload(SceneStore& st, cudaStream_t s) {
             pairs[4 * n + 2] = make_float4(lo.z, lh.z, ro.z, rh.z);
             pairs[4 * n + 3] = make_float4(int_bits(code(leaf_of(l), (int)l)), int_bits(code(leaf_of((size_t)r), r)), int_bits(r), 0.0f);
         }
-        st.scene.use_pairs = !full_binary ? 0 : empty_leaf ? 1 : nested ? 3 : 2;
+        st.scene.use_pairs = !full_binary ? 0 : empty_leaf ? 1 : deep ? 2 : 3;
         st.scene.pair_stack = 8;
         CUDA_TRY(upload(st.pairs, pairs, s));
         CUDA_TRY(cudaStreamSynchronize(s));

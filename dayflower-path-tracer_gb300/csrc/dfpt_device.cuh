@@ -795,34 +795,26 @@ __device__ __forceinline__ int2* walk_stack() {
 // record (-1: none of this mesh is closer).
 //
 // A record gives both children's boxes in two 32-byte loads and six packed FMAs. Both children
-// accepted: one is pushed with its key (see mesh_walk_pair_compact: key < closest is its box test at
-// any later time) and the other entered.
-// Order. The reference visits in preorder, and one of its box tests depends on that: a box that
-// holds the ray's origin is entered only while its exit lies before the closest hit so far. Such
-// boxes form the top of the tree (a box around the origin has such a parent; scene_upload checks
-// that children lie in their parents), and below one the origin lies outside of lies no other.
-// Inside the subtrees that the ray enters from outside, an unvisited box can only hold hits beyond
-// its entry, so their order does not change the closest hit: there (both children's entries ahead of
-// the origin) the nearer child goes first, everywhere else the left one. Of two triangles hit at
-// the same distance - a ray through their shared edge - the one first in preorder is kept, as the
-// reference keeps it. The strict set, whose ids equal the reference's bit for bit, keeps preorder
-// throughout.
+// accepted: the right one is pushed with its key (see mesh_walk_pair_compact: key < closest is its box
+// test at any later time) and the left one entered, so every box and triangle is tested in preorder,
+// with the closest distance of that moment: the counting walks' hits.
+// The order is part of the result. Rays through an edge that two triangles share hit both, an ulp apart
+// or at one distance, and often meet the second one's box exactly at the hit, where the box test drops
+// it: the triangle visited first is kept. The nearer child first where both lie ahead of the origin
+// keeps the other one - of 3 in 10 rays aimed along shared edges, one in 2.4 million of mesh_scene's -
+// and no bound on the slabs' rounding mends that for all rays: a triangle's own distance is as far off as
+// the ray grazes it. It would save 10 of 52 box tests of a camera ray, and 2 % of a bounce ray's.
 //
 // Shape of the loop: a lane steps through inner nodes until it holds a leaf or is done; the lanes of
 // a warp meet there and test their leaves together. One loop with a branch per node kind, which lets
-// descending lanes run ahead, measured 22.6 ms against 20.9 for a 32-pass 1080p mesh_scene step
-// (any hit 10.5 against 6.9), and a vote per step 24.8 (7.3).
+// descending lanes run ahead, and a vote per step were both slower (8 and 19 % of closest hits, 52 and
+// 6 % of any hits).
 //
 // What bounds it: instruction issue at the lanes that divergence leaves (the compact pair walk: 75 %
 // of issue slots at 16 lanes per instruction on camera rays, 67 % at 9 on bounce rays) and the
 // load/store pipe (75 % of its wavefronts); hence wide loads, packed FMAs, no counters, the object-
 // space ray kept from primitive to primitive and no overflow logic on the common path. Closest hits
 // of that step 30.2 -> 20.9 ms; its shadow rays, from the threaded walk, 8.1 -> 6.9.
-#ifdef DFPT_STRICT_MATH
-#define DFPT_NEAR_FIRST false
-#else
-#define DFPT_NEAR_FIRST true
-#endif
 template <bool ANY, int NT>
 __device__ __forceinline__ bool pair_walk(const DevScene& S, int root, float ox, float oy, float oz, float dx, float dy, float dz,
                                           const SlabRay2& sr, float& closest, int& best) {
@@ -870,9 +862,7 @@ __device__ __forceinline__ bool pair_walk(const DevScene& S, int root, float ox,
             const int lc = __float_as_int(e.x), rc = __float_as_int(e.y);
             code = al ? lc : rc;
             if (al && ar) {
-                const bool swap = DFPT_NEAR_FIRST && !ANY && rmin > 0.001f && rmin < lmin;
-                const int2 later = swap ? make_int2(lc, __float_as_int(lkey)) : make_int2(rc, __float_as_int(rkey));
-                if (swap) code = rc;
+                const int2 later = make_int2(rc, __float_as_int(rkey));
                 if (top < DFPT_WALK_STACK) stk[top * NT] = later;
                 else deep[top - DFPT_WALK_STACK] = later;
                 ++top;
@@ -891,7 +881,7 @@ __device__ __forceinline__ bool pair_walk(const DevScene& S, int root, float ox,
                     closest = t;
                     return true;
                 }
-            } else if (t < closest || (t == closest && k < best)) {
+            } else if (t < closest) {
                 closest = t;
                 best = k;
             }

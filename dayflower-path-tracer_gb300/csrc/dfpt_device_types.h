@@ -34,8 +34,8 @@ struct DevScene {
                             // child's index (inner), ~(first triangle) (leaf) or INT_MIN (empty leaf)
     int use_pairs;          // 1: every mesh BVH is a full binary tree, so pair records describe the walk;
                             // 2: the same, and no leaf is empty (the compact pair walk's condition);
-                            // 3: the same, children and triangles lie in their boxes and no tree is deeper
-                            // than DFPT_WALK_DEPTH (the packed pair walk's condition)
+                            // 3: the same, and no tree is deeper than DFPT_WALK_DEPTH (the packed pair
+                            // walk's condition)
     int flat;               // no primitive is a mesh
     const int4* prim_walk;  // {shape type, shape offset, record index, first primitive of the run with this matrix}
     int pair_stack;         // entries of the compact pair walk's stack in use (1..8; 8 unless a test lowers it)

@@ -61,7 +61,6 @@ struct Derived {
     // Primitive culling (see build_culling): BVH nodes, leaf lists, unbounded primitives, boxes.
     std::vector<float4> cull_nodes, prim_box;
     std::vector<int> cull_prims, always;
-    bool nested = true;  // every mesh triangle lies in its leaf's box
     int bounded = 0;  // primitives with a world box
     float4 bounds_lo = make_float4(-1.0e4f, -1.0e4f, -1.0e4f, 0), bounds_hi = make_float4(1.0e4f, 1.0e4f, 1.0e4f, 0);
 };

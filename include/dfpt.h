@@ -205,9 +205,8 @@ int dfpt_read_hits(dfpt_handle* handle, int32_t* primitive_offset, int32_t* shap
  * BVH nodes visited and triangles tested (summed over all segments), then the nodes and the
  * triangles of the closest-hit segments alone. */
 int dfpt_read_counters(dfpt_handle* handle, uint64_t* counters6);
-/* Enables (1) or disables (0, the default) the traversal counters; counting costs atomics, and the
- * walks then visit nodes in the reference's order (uncounted closest-hit walks may take the nearer
- * child first where that cannot change the hit). */
+/* Enables (1) or disables (0, the default) the traversal counters; counting costs atomics, and
+ * configurations 16 and 17 then run other kernels with the same visits and hits. */
 int dfpt_set_counting(dfpt_handle* handle, int32_t enabled);
 
 /* Per-kernel timing of the last dfpt_render call: when enabled, passes are issued as direct
@@ -220,9 +219,8 @@ int dfpt_read_profile(dfpt_handle* handle, double* ms_by_kind10, int32_t* launch
 /* Launch tuning (no reference counterpart; results never depend on it). Keys:
  *   "trace_config"      traversal kernel configuration (walk variant x block size x resident
  *                       blocks per SM, 0..N-1, N readable as "trace_configs"); every configuration
- *                       finds the same hits, and visits the same nodes in the same order when
- *                       they are counted (default 16, a walk over records of child pairs, the
- *                       autotuner's usual pick);
+ *                       visits the same nodes in the same order (default 16, a walk over records
+ *                       of child pairs, the autotuner's usual pick);
  *   "shadow_config"     the configuration of the sun shadow-ray (any-hit) launches; -1 (default)
  *                       the trace_config's (any hit is the same hit-or-miss in every walk order);
  *   "pair_stack"        stack entries of the compact pair walk (1..8, default 8); fewer entries
