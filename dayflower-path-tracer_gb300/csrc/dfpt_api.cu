@@ -1288,7 +1288,9 @@ int scene_upload(SceneStore& st, cudaStream_t s) {
         std::vector<float4> pairs(4 * nn, make_float4(0, 0, 0, 0));
         bool full_binary = true, empty_leaf = false;
         bool deep = false;  // a tree deeper than the packed pair walk's stack
-        std::vector<uint8_t> depth(nn, 0);  // roots at 0; a child comes after its parent in preorder
+        // Levels below the root: roots at 0; a child comes after its parent. The most of all nodes that name
+        // it a child: next pointers may skip nodes, and a skipped one may name a node of the walk's tree.
+        std::vector<uint8_t> depth(nn, 0);
         auto next_of = [&](size_t n) { return float_bits_int(d.nodes[2 * n].w); };
         auto leaf_of = [&](size_t n) { return float_bits_int(d.nodes[2 * n + 1].w); };
         for (size_t n = 0; n < nn && full_binary; ++n) {
@@ -1299,7 +1301,7 @@ int scene_upload(SceneStore& st, cudaStream_t s) {
             if (l >= nn || r < 0 || (size_t)r >= nn || next_of((size_t)r) != next_of(n)) { full_binary = false; break; }
             const float4 lo = d.nodes[2 * l], lh = d.nodes[2 * l + 1], ro = d.nodes[2 * (size_t)r], rh = d.nodes[2 * (size_t)r + 1];
             deep = deep || depth[n] >= DFPT_WALK_DEPTH;
-            depth[l] = depth[(size_t)r] = (uint8_t)std::min(depth[n] + 1, DFPT_WALK_DEPTH);
+            for (size_t child : {l, (size_t)r}) depth[child] = std::max(depth[child], (uint8_t)std::min(depth[n] + 1, DFPT_WALK_DEPTH));
             auto code = [&](int leaf, int node) { return leaf == -1 ? node : leaf == -2 ? INT32_MIN : ~leaf; };
             pairs[4 * n] = make_float4(lo.x, lo.y, lh.x, lh.y);
             pairs[4 * n + 1] = make_float4(ro.x, ro.y, rh.x, rh.y);

@@ -68,3 +68,57 @@ def test_rays_along_shared_edges_keep_the_preorder_hit(width, height, flat):
         assert (counted[2] >= 0).sum() > width * height // 2, "the mesh does not fill the image"
         for a, b in zip(uncounted, counted):
             assert np.array_equal(a, b), (renderer, int((np.asarray(a) != np.asarray(b)).sum()))
+
+
+def _skipped_parent(lefts, chain):
+    """A mesh tree in which a skipped node names the node that a chain of `chain` left children hangs from its
+    child, `lefts` + 1 levels above that node's place in the walk's tree."""
+    from dfpt import scene as sc, synthetic
+
+    count = lefts + chain + 3
+    corners = []
+    for k in range(count):
+        z, s = 0.02 * k, 2.0 * (1.0 - k / (count + 10.0))
+        corners += [(-s + 0.3, -s + 0.7, z), (s + 0.3, -0.8 * s + 0.7, z), (0.1 * s + 0.3, s + 0.7, z - 0.05)]
+    b, black = _builder(72, 56)
+    positions, indices = np.asarray(corners), np.arange(3 * count, dtype=np.int32).reshape(-1, 3)
+    normals = synthetic.vertex_normals(positions, indices)
+    mesh = b.mesh(positions, indices, normals, np.zeros((len(positions), 2)), synthetic.tangents_for(normals))
+    b.primitive(mesh, b.surface(sc.LAMBERTIAN, b.constant(0.7, 0.6, 0.5), black, black))
+    scene = b.compile("skipped")
+    point = scene.point3fs.reshape(-1)
+    tris = np.arange(0, scene.triangles.size, 12)
+    tri_corners = np.stack([[point[scene.triangles[t + v]:scene.triangles[t + v] + 3] for v in range(3)] for t in tris])
+    lo, hi = tri_corners.min((0, 1)) - 0.1, tri_corners.max((0, 1)) + 0.1  # one box for every node
+    box = [point.size, point.size + 3]
+    # Nodes in order: (kind, name, next name). Inner nodes' left child is the node behind them.
+    nodes = [("inner", f"i{k}", f"r{k - 1}" if k else None) for k in range(lefts)]
+    after = f"r{lefts - 1}"
+    nodes += [("inner", "top", after), ("leaf", "a", "x0"), ("inner", "skipped", after), ("leaf", "o", "x0")]
+    nodes += [("inner", f"x{k}", f"y{k - 1}" if k else after) for k in range(chain)]
+    nodes += [("leaf", "bottom", f"y{chain - 1}")] + [("leaf", f"y{k}", f"y{k - 1}" if k else after) for k in reversed(range(chain))]
+    nodes += [("leaf", f"r{k}", f"r{k - 1}" if k else None) for k in reversed(range(lefts))]
+    at, offsets = 0, {}
+    for kind, name, _ in nodes:
+        offsets[name] = at
+        at += 5 if kind == "inner" else 6
+    out, tri = [], iter(tris)
+    for kind, name, following in nodes:
+        nxt = -1 if following is None else offsets[following]
+        out += [1, nxt, *box, offsets[name] + 5] if kind == "inner" else [2, nxt, *box, 1, int(next(tri))]
+    scene.primitives[3 + 1] = scene.bounding_volume_hierarchies.size
+    scene.bounding_volume_hierarchies = np.concatenate([scene.bounding_volume_hierarchies, np.asarray(out, np.int32)])
+    scene.point3fs = np.concatenate([point, lo, hi]).astype(np.float32)
+    params = dict(renderer_type=2, pt_ray_depth_maximum=3, pt_ray_depth_russian_roulette=3, tone_mapper_type=2)
+    return scene, sc.SkyState((0.5, 0.7, 0.4), 2.5), params
+
+
+@pytest.mark.parametrize("lefts,chain", [(3, 5), (10, 53), (10, 60), (40, 60)])
+def test_depth_of_trees_with_skipped_nodes(lefts, chain):
+    """A ray through every box has an entry pending per level: trees deeper than the stack keep another walk."""
+    scene, sky, params = _skipped_parent(lefts, chain)
+    for renderer in (1, 2, 3):
+        uncounted, counted = (_hits(scene, sky, dict(params, renderer_type=renderer), 72, 56, c) for c in (False, True))
+        assert (counted[2] >= 0).any()
+        for a, b in zip(uncounted, counted):
+            assert np.array_equal(a, b)
