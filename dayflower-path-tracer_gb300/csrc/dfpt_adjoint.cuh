@@ -211,12 +211,15 @@ __device__ void sun_rim_tan(const DevScene& S, const DevParams& P, uint32_t pixe
 // Per-block gradient accumulation: per-primitive entries in shared memory (float, one launch) when
 // they fit, else straight into row 0 with double atomics; the four sky entries in registers.
 //
-// A vertex's seven entries are gathered in registers and added by the warp together: lanes of one
-// primitive sum theirs with shuffles and one lane adds the sums. A float atomic on shared memory is
-// a compare-and-swap loop, and a wave's neighbouring lanes mostly hit one primitive (at bounce 0 the
+// Shared mode: a vertex's seven entries are gathered in registers and added by the warp together: lanes
+// of one primitive sum theirs with shuffles and one lane adds the sums. A float atomic on shared memory
+// is a compare-and-swap loop, and a wave's neighbouring lanes mostly hit one primitive (at bounce 0 the
 // samples of one or two pixels), so lane by lane the loops ran up to 32 times for each entry: the
 // backward of 16 passes at 512 x 512 over 257 primitives took 5.8 ms, 4.0 now.
 // Groups of fewer than 4 lanes add on their own.
+// Atomic mode: every term is added on its own, in double; a sum of lanes in float would lose what the
+// double entries are there to keep where large terms cancel, and double atomics on global memory run in
+// L2 without a loop.
 struct GradAcc {
     float* sh;     // shared [P * 7] or null
     double* row;   // this block's row (shared mode) / row 0 (atomic mode)
@@ -225,7 +228,7 @@ struct GradAcc {
         if (sh) atomicAdd(sh + prim * DFPT_DIFF_PER_PRIM + k, v);
         else atomicAdd(row + prim * DFPT_DIFF_PER_PRIM + k, (double)v);
     }
-    // All 32 lanes call it; prim < 0: no vertex.
+    // Shared mode. All 32 lanes call it; prim < 0: no vertex.
     __device__ __forceinline__ void add_warp(int prim, const float g[DFPT_DIFF_PER_PRIM]) {
         const unsigned same = __match_any_sync(0xFFFFFFFFu, prim);
         const int lane = threadIdx.x & 31;
@@ -295,8 +298,12 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
     GRID_STRIDE_UNIFORM(i, n) {
         bool emit_next = false;
         float4 no = make_float4(0, 0, 0, 0), nd = make_float4(0, 0, 0, 0);
-        int vertex = -1;  // its primitive, and what it adds to the primitive's entries
+        int vertex = -1;  // its primitive, and (shared mode) what it adds to the primitive's entries
         float g[DFPT_DIFF_PER_PRIM] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        auto put = [&](int k, float v) {
+            if constexpr (SHARED) g[k] += v;
+            else acc.add(vertex, k, v);
+        };
         if (i < n) {
             const float4 o4 = B.q_o[qi][i], d4 = B.q_d[qi][i];
             const int path = __float_as_int(o4.w);
@@ -344,9 +351,9 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                 // Emission.
                 Lu.x += T.x * er; Lu.y += T.y * eg; Lu.z += T.z * eb;
                 vertex = h.prim;
-                g[3] = w.x * T.x;
-                g[4] = w.y * T.y;
-                g[5] = w.z * T.z;
+                put(3, w.x * T.x);
+                put(4, w.y * T.y);
+                put(5, w.z * T.z);
                 // Sun sample (same draws as the forward; visibility from the forward's bits).
                 if ((material == DFPT_MATERIAL_CLEAR_COAT || material == DFPT_MATERIAL_LAMBERTIAN || material == DFPT_MATERIAL_PHONG) &&
                     P.sun_active == 1) {
@@ -358,9 +365,9 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                     if (sun_sample(P, s.px, s.py, s.pz, wx, wy, wz, u, v, lx, ly, lz, dot1) && seen) {
                         const float k = dot1 * INV_PI;
                         Lu.x += T.x * (ar * 1.0f * k); Lu.y += T.y * (ag * 1.0f * k); Lu.z += T.z * (ab * 1.0f * k);
-                        g[0] = w.x * T.x * tr * k;
-                        g[1] = w.y * T.y * tg * k;
-                        g[2] = w.z * T.z * tb * k;
+                        put(0, w.x * T.x * tr * k);
+                        put(1, w.y * T.y * tg * k);
+                        put(2, w.z * T.z * tb * k);
                         g_forward = c * dot1;
                     }
                     sun_rim_tan(S, P, pixel, pass, bounce, s.px, s.py, s.pz, wx, wy, wz, c, g_forward, gsky);
@@ -382,12 +389,12 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                     // Radiance of the later vertices (every term carries this vertex's factors).
                     const float lr = Lt.x - Lu.x, lg = Lt.y - Lu.y, lb = Lt.z - Lu.z;
                     if (sct.albedo) {
-                        if (a0r != 0.0f) g[0] += w.x * lr * tr / a0r;
-                        if (a0g != 0.0f) g[1] += w.y * lg * tg / a0g;
-                        if (a0b != 0.0f) g[2] += w.z * lb * tb / a0b;
+                        if (a0r != 0.0f) put(0, w.x * lr * tr / a0r);
+                        if (a0g != 0.0f) put(1, w.y * lg * tg / a0g);
+                        if (a0b != 0.0f) put(2, w.z * lb * tb / a0b);
                     }
                     if (material == DFPT_MATERIAL_PHONG && sct.phong_ct > 0.0f)
-                        g[6] = (w.x * lr + w.y * lg + w.z * lb) * (1.0f / (exponent + 1.0f) + logf(sct.phong_ct));
+                        put(6, (w.x * lr + w.y * lg + w.z * lb) * (1.0f / (exponent + 1.0f) + logf(sct.phong_ct)));
                     emit_next = true;
                     no = make_float4(sct.o.x, sct.o.y, sct.o.z, __int_as_float(path));
                     nd = make_float4(sct.d.x, sct.d.y, sct.d.z, 0.0f);
@@ -397,7 +404,7 @@ __global__ void __launch_bounds__(256) k_shade_adj(DevScene S, const DevParams* 
                 B.rng[path] = rng.state;
             }
         }
-        acc.add_warp(vertex, g);
+        if constexpr (SHARED) acc.add_warp(vertex, g);
         const int slot = warp_push(B.counts + bounce + 1, emit_next);
         if (slot >= 0) {
             B.q_o[qi ^ 1][slot] = no;
