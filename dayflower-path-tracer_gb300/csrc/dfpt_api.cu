@@ -871,7 +871,7 @@ int wide_prepare(dfpt_handle* h) {
         if (!h->w_vis.p) CUDA_TRY(h->w_vis.alloc((size_t)h->wide_capacity));
         B.vis = h->w_vis.p;
         B.diff_L = h->pass.diff_L; B.diff_vis = h->pass.diff_vis; B.diff_dldi = h->pass.diff_dldi;
-        B.diff_rows = h->pass.diff_rows; B.diff_row_len = h->pass.diff_row_len;
+        B.diff_rows = h->pass.diff_rows; B.diff_row_len = h->pass.diff_row_len; B.diff_row_count = h->pass.diff_row_count;
     }
     if (B.sorted_queues && !h->w_s2_o.p) {
         CUDA_TRY(h->w_s2_o.alloc(h->wide_shadow));
@@ -2059,7 +2059,7 @@ int dfpt_diff_forward(dfpt_handle* h, const dfpt_diff_params* dp, int32_t spp, f
     }
     DevPass& B = h->pass;
     B.vis = h->vis.p; B.diff_L = h->diff_L.p; B.diff_vis = h->diff_vis.p; B.diff_dldi = h->diff_dldi.p;
-    B.diff_rows = h->diff_rows.p; B.diff_row_len = row_len;
+    B.diff_rows = h->diff_rows.p; B.diff_row_len = row_len; B.diff_row_count = rows;
     h->graph_valid = false;
     h->wide_graph_valid = false;  // the pass record changed
     h->diff_on = true;

@@ -160,6 +160,7 @@ struct DevPass {
     const float* diff_dldi;    // 3 per pixel: dLoss/dImage (rgb), as the caller passed it
     double* diff_rows;         // per block of the adjoint kernels: gradient partials
     int diff_row_len;          // primitives x 7 + 4
+    int diff_row_count;        // rows: the most blocks that the adjoint kernels may have
     // Ray binning between bounces (wide passes): with sorted_queues set, shading writes queue 1,
     // the binning pass moves it to queue 0 in bin order, and every bounce reads queue 0.
     int sorted_queues;

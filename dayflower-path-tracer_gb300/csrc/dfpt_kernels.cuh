@@ -2411,16 +2411,17 @@ template <bool BATCH>
 static void launch_shade_adj_t(const LaunchCtx& c, int bounce) {
     const DevBatch Q = BATCH ? *c.batch : DevBatch{};
     const size_t bytes = (size_t)c.scene->primitive_count * DFPT_DIFF_PER_PRIM * sizeof(float);
-    // One row per block of c.grid blocks; no more than are resident (at 128 registers 2 per SM, where
-    // c.grid's 3 left a second round half empty).
-    if (bytes <= 44 * 1024) k_shade_adj<BATCH, true><<<std::min(c.grid, resident_grid(k_shade_adj<BATCH, true>, 256, bytes)), 256, bytes, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
-    else k_shade_adj<BATCH, false><<<std::min(c.grid, resident_grid(k_shade_adj<BATCH, false>, 256)), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
+    // A row per block; no more blocks than are resident (at 128 registers 2 per SM, where c.grid's 3 left a
+    // second round half empty).
+    const int rows = c.pass->diff_row_count;
+    if (bytes <= 44 * 1024) k_shade_adj<BATCH, true><<<std::min(rows, resident_grid(k_shade_adj<BATCH, true>, 256, bytes)), 256, bytes, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
+    else k_shade_adj<BATCH, false><<<std::min(rows, resident_grid(k_shade_adj<BATCH, false>, 256)), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
 }
 template <bool BATCH>
 static void launch_final_adj_t(const LaunchCtx& c, int bounce) {
     // Per-lane walks (variant 1 prefetches); one block per gradient row.
     const DevBatch Q = BATCH ? *c.batch : DevBatch{};
-    k_final_adj<BATCH, 1><<<c.grid, 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
+    k_final_adj<BATCH, 1><<<std::min(c.grid, c.pass->diff_row_count), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
 }
 #ifndef DFPT_ONE_SCENE
 static void launch_shade_adj(const LaunchCtx& c, int bounce) { launch_shade_adj_t<false>(c, bounce); }

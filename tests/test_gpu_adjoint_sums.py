@@ -36,3 +36,31 @@ def test_gradients_of_many_primitives_are_summed_in_double(spp):
     k.dispose()
     assert np.array_equal(emission[0], weights.astype(np.float64).sum((0, 1)))
     assert not emission[1:].any()
+
+
+@pytest.mark.parametrize("strict_first", [False, True])
+def test_kernel_set_switched_between_forward_and_backward(strict_first):
+    """The gradient rows belong to the forward; the backward's launches, whose grids follow the kernel set
+    selected then, take no more blocks than there are rows. Gradients as without the switch: the replay is
+    the same, pass by pass or in waves (rtol 1e-4 per group, what the order of float sums leaves there)."""
+    from dfpt import synthetic
+    from dfpt.diff import DiffRenderer
+    from dfpt.kernel import RendererKernel
+    from dfpt.scene import SkyState
+
+    scene, params, (w, h), truth, start = synthetic.inverse_scene(seed=4, width=160, height=120, count=25)
+    weights = np.random.default_rng(2).normal(size=(h, w, 3)).astype(np.float32)
+    out = []
+    for switched in (False, True):
+        k = RendererKernel(scene, SkyState((0.3, 0.9, 0.25), 2.5), dict(params, seed=5))
+        k.update(w, h)
+        k.set_strict(strict_first)
+        d = DiffRenderer(k)
+        d.forward(start["albedo"], None, start["phong_exponent"], 2.5, (0.3, 0.9, 0.25), 4)
+        k.set_strict(strict_first != switched)
+        out.append(d.backward(weights))
+        k.dispose()
+    for key in ("albedo", "emission", "phong_exponent", "sun_direction"):
+        a, b = (np.asarray(g[key]).ravel() for g in out)
+        assert np.linalg.norm(a) > 0
+        assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(a), key
