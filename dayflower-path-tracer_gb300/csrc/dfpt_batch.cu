@@ -183,8 +183,8 @@ int batch_prepare(dfpt_batch* b) {
     B.sort_count_shadow = b->sort_bins.p ? b->sort_bins.p + 2 * DFPT_SORT_BINS : nullptr;
     B.sort_partials = b->sort_bins.p ? b->sort_bins.p + 3 * DFPT_SORT_BINS : nullptr;
     if (b->stores.size() > 1) {
-        B.sort_ray_bits = sort_bits(b->capacity, 8 * 128, 4, 12);
-        B.sort_shadow_bits = sort_bits(b->capacity, 8, 6, 18);
+        B.sort_ray_bits = sort_bits(b->capacity, DFPT_BATCH_SCENES * DFPT_BATCH_RAY_DIRS, 4, DFPT_BATCH_RAY_CELL_BITS);
+        B.sort_shadow_bits = sort_bits(b->capacity, DFPT_BATCH_SCENES, 6, DFPT_BATCH_SHADOW_CELL_BITS);
     } else {
         B.sort_ray_bits = sort_bits(b->capacity, DFPT_RAY_DIRS, 4, DFPT_RAY_CELL_BITS);
         B.sort_shadow_bits = sort_bits(b->capacity, 1, 6, DFPT_SHADOW_CELL_BITS);

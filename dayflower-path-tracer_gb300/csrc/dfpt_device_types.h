@@ -175,13 +175,24 @@ struct DevPass {
 // of sort_ray_bits bits, a shadow ray's the cell of a grid of sort_shadow_bits bits (multiples of 3: an
 // equal split over the axes). Waves of several scenes: 3 bits of the scene's place in the wave above
 // either, the direction then in 7 bits. The grids follow the slots of a launch (sort_bits below), up
-// to DFPT_RAY_CELL_BITS and DFPT_SHADOW_CELL_BITS (12 and 18 with several scenes); every key stays
+// to DFPT_RAY_CELL_BITS and DFPT_SHADOW_CELL_BITS (the BATCH ones with several scenes); every key stays
 // below DFPT_SORT_BINS. The scan runs over chunks of 1024 bins.
 #define DFPT_RAY_CELL_BITS 15
 #define DFPT_SHADOW_CELL_BITS 21
+#define DFPT_BATCH_RAY_CELL_BITS 12
+#define DFPT_BATCH_SHADOW_CELL_BITS 18
 #define DFPT_RAY_DIRS 96
+#define DFPT_BATCH_SCENES 8      // keys of a scene's place in the wave
+#define DFPT_BATCH_RAY_DIRS 128  // 96 directions in 7 bits
 #define DFPT_SORT_BINS (1 << 22)
 #define DFPT_SORT_CHUNKS (DFPT_SORT_BINS / 1024)
+static_assert(((long long)DFPT_RAY_DIRS << DFPT_RAY_CELL_BITS) <= DFPT_SORT_BINS && (1ll << DFPT_SHADOW_CELL_BITS) <= DFPT_SORT_BINS &&
+                  ((long long)DFPT_BATCH_SCENES * DFPT_BATCH_RAY_DIRS << DFPT_BATCH_RAY_CELL_BITS) <= DFPT_SORT_BINS &&
+                  ((long long)DFPT_BATCH_SCENES << DFPT_BATCH_SHADOW_CELL_BITS) <= DFPT_SORT_BINS,
+              "every bin key lies in the bin array, whatever the grids");
+static_assert(DFPT_RAY_CELL_BITS % 3 == 0 && DFPT_SHADOW_CELL_BITS % 3 == 0 && DFPT_BATCH_RAY_CELL_BITS % 3 == 0 &&
+                  DFPT_BATCH_SHADOW_CELL_BITS % 3 == 0 && DFPT_SHADOW_CELL_BITS <= 21 && DFPT_RAY_DIRS <= DFPT_BATCH_RAY_DIRS,
+              "cells come from a 128^3 grid, the same number of bits per axis");
 
 // The grid's bits for bins of `per_cell` keys a cell: as fine as leaves `rays` rays a bin when each of
 // `slots` slots emits one, at least 3, at most `most`. The scan reads and writes every bin, so bins that

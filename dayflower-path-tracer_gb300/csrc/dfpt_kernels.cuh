@@ -648,8 +648,9 @@ __device__ __forceinline__ WavePixels wave_pixels(const DevBatch& Q) {
     w.rng_pass = (uint32_t)(w.first + Q.wave_base[2]);
     return w;
 }
-// Slot -> pixel and place among the pixel's passes, pixel-major (at most one too high before the check:
-// slots stay below 2^27 and passes at most 64).
+// Slot -> pixel and place among the pixel's passes, pixel-major. The quotient is at most one too high before
+// the check, for any number of passes: the inverse exceeds 2^32 / passes by less than one, and slots stay
+// below 2^32.
 __device__ __forceinline__ void pixel_of_wave_slot(const WavePixels& w, unsigned slot, unsigned& pixel, unsigned& j) {
     pixel = w.passes > 1u ? __umulhi(slot, w.inverse) : slot;
     int r = (int)(slot - pixel * w.passes);
@@ -1030,12 +1031,12 @@ __device__ __forceinline__ int plain_ray_bin(const DevScene& S, float4 o, float4
 __device__ __forceinline__ int ray_bin_in_wave(const DevBatch& Q, int first, float4 o, float4 d, int bits) {
     const int sid = __float_as_int(d.w);
     const int bin = plain_ray_bin(Q.scenes[sid], o, d, bits);
-    return Q.n_scenes == 1 ? bin : (((sid - first) & 7) << (bits + 7)) | bin;
+    return Q.n_scenes == 1 ? bin : ((((sid - first) & (DFPT_BATCH_SCENES - 1)) * DFPT_BATCH_RAY_DIRS) << bits) | bin;
 }
 __device__ __forceinline__ int shadow_bin_in_wave(const DevBatch& Q, int first, float4 o, float4 d, int bits) {
     const int sid = __float_as_int(d.w);
     const int bin = cell_bits(Q.scenes[sid], o, bits);
-    return Q.n_scenes == 1 ? bin : (((sid - first) & 7) << bits) | bin;
+    return Q.n_scenes == 1 ? bin : (((sid - first) & (DFPT_BATCH_SCENES - 1)) << bits) | bin;
 }
 
 // Bin counts with one atomic per distinct bin of a warp.
@@ -2050,9 +2051,9 @@ static int launch_sort_scan(const LaunchCtx& c, int* counts, long long keys) {
     return 3;
 }
 static long long ray_keys(const LaunchCtx& c, int scenes) {
-    return (scenes > 1 ? 8 * 128ll : (long long)DFPT_RAY_DIRS) << c.pass->sort_ray_bits;
+    return (scenes > 1 ? (long long)DFPT_BATCH_SCENES * DFPT_BATCH_RAY_DIRS : (long long)DFPT_RAY_DIRS) << c.pass->sort_ray_bits;
 }
-static long long shadow_keys(const LaunchCtx& c, int scenes) { return (scenes > 1 ? 8ll : 1ll) << c.pass->sort_shadow_bits; }
+static long long shadow_keys(const LaunchCtx& c, int scenes) { return (scenes > 1 ? (long long)DFPT_BATCH_SCENES : 1ll) << c.pass->sort_shadow_bits; }
 
 __global__ void __launch_bounds__(256) k_sort_scatter(DevBatch Q, DevPass B, int bounce) {
     const int n = B.counts[bounce + 1];
