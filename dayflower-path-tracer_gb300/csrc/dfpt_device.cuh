@@ -277,33 +277,9 @@ __device__ __forceinline__ float isect_sphere(float ox, float oy, float oz, floa
     return INF;
 }
 
-// Moller-Trumbore with the reference's tolerances; e0 = b - a and e1 = c - a precomputed.
-__device__ __forceinline__ float isect_triangle(float ox, float oy, float oz, float dx, float dy, float dz, float4 a, float4 e0, float4 e1, float tmax) {
-    const float v0x = dy * e1.z - dz * e1.y;
-    const float v0y = dz * e1.x - dx * e1.z;
-    const float v0z = dx * e1.y - dy * e1.x;
-    const float det = e0.x * v0x + e0.y * v0y + e0.z * v0z;
-    float t = INF;
-    if (det < -0.0001f || det > 0.0001f) {
-        const float inv = 1.0f / det;
-        const float v1x = ox - a.x, v1y = oy - a.y, v1z = oz - a.z;
-        const float u = (v1x * v0x + v1y * v0y + v1z * v0z) * inv;
-        if (u >= 0.0f && u <= 1.0f) {
-            const float v2x = v1y * e0.z - v1z * e0.y;
-            const float v2y = v1z * e0.x - v1x * e0.z;
-            const float v2z = v1x * e0.y - v1y * e0.x;
-            const float v = (dx * v2x + dy * v2y + dz * v2z) * inv;
-            t = v >= 0.0f && u + v <= 1.0f ? (e1.x * v2x + e1.y * v2y + e1.z * v2z) * inv : 0.001f;
-            t = t > 0.001f && t < tmax ? t : INF;
-        }
-    }
-    return t;
-}
-
-// a . b with the roundings that contraction gives the three products written out in the shape tests
-// above; the forms below are those tests with every fused operation named, so that they give the
-// same floats wherever they are inlined (which product of a sum is fused depends on where its operands
-// come from).
+// a . b, and a * b - c * d, with the roundings that contraction gives the products where they are written out.
+// The forms below are with every fused operation named, so that they give the same floats wherever they are
+// inlined: which product of a sum is fused depends on where its operands come from.
 __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz) {
 #ifdef DFPT_FMA_SLABS
     return __fmaf_rn(az, bz, __fmaf_rn(ax, bx, __fmul_rn(ay, by)));
@@ -311,6 +287,41 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
     return ax * bx + ay * by + az * bz;
 #endif
 }
+__device__ __forceinline__ float det2(float a, float b, float c, float d) {
+#ifdef DFPT_FMA_SLABS
+    return __fmaf_rn(a, b, -__fmul_rn(c, d));
+#else
+    return a * b - c * d;
+#endif
+}
+// Moller-Trumbore with the reference's tolerances; e0 = b - a and e1 = c - a precomputed.
+__device__ __forceinline__ float isect_triangle(float ox, float oy, float oz, float dx, float dy, float dz, float4 a, float4 e0, float4 e1, float tmax) {
+    const float v0x = det2(dy, e1.z, dz, e1.y);
+    const float v0y = det2(dz, e1.x, dx, e1.z);
+    const float v0z = det2(dx, e1.y, dy, e1.x);
+    const float det = dot3(e0.x, e0.y, e0.z, v0x, v0y, v0z);
+    float t = INF;
+    if (det < -0.0001f || det > 0.0001f) {
+        const float inv = 1.0f / det;
+        const float v1x = ox - a.x, v1y = oy - a.y, v1z = oz - a.z;
+        const float su = dot3(v1x, v1y, v1z, v0x, v0y, v0z), u = su * inv;
+        if (u >= 0.0f && u <= 1.0f) {
+            const float v2x = det2(v1y, e0.z, v1z, e0.y);
+            const float v2y = det2(v1z, e0.x, v1x, e0.z);
+            const float v2z = det2(v1x, e0.y, v1y, e0.x);
+            const float v = dot3(dx, dy, dz, v2x, v2y, v2z) * inv;
+#ifdef DFPT_FMA_SLABS
+            const float uv = __fmaf_rn(su, inv, v);
+#else
+            const float uv = u + v;
+#endif
+            t = v >= 0.0f && uv <= 1.0f ? dot3(e1.x, e1.y, e1.z, v2x, v2y, v2z) * inv : 0.001f;
+            t = t > 0.001f && t < tmax ? t : INF;
+        }
+    }
+    return t;
+}
+
 __device__ __forceinline__ float isect_plane_f(float ox, float oy, float oz, float dx, float dy, float dz, float4 a, float4 n, float tmax) {
     const float dp = dot3(n.x, n.y, n.z, dx, dy, dz);
     if (dp < 0.0f || dp > 0.0f) {
@@ -1061,7 +1072,7 @@ __device__ __forceinline__ float box_entry(float4 lo, float4 hi, float ox, float
 }
 
 // box_entry for the packed walks: the same slab products two at a time, from one 32-byte load of a box.
-// A direction component below 1e-20 takes the reciprocal +-1e30, which sends a slab that does not
+// A direction component below 1e-30 takes the reciprocal +-1e30, which sends a slab that does not
 // hold the origin beyond any hit and leaves one that does unbounded.
 struct CullRay {
     float2 oxy, oz, ixy, iz;  // the origin negated
