@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256) k_final_adj(DevScene S, const DevParams* 
     const int n_prim_entries = S.primitive_count * DFPT_DIFF_PER_PRIM;
     const float inv_spp = 1.0f / (float)P.diff_spp;
     float gsky[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    WARP_DYNAMIC(i, n, B.counts + DFPT_COUNTS_FETCH + bounce) {
+    WARP_DYNAMIC(i, n, S.terrain, B.counts + DFPT_COUNTS_FETCH + bounce) {
         TraceStats st{0, 0};
         const bool valid = i < n;
         float4 o = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 1, 0);

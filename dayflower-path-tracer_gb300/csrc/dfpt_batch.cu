@@ -219,8 +219,8 @@ int batch_prepare(dfpt_batch* b) {
     // One launch walks every scene's rays; the packed pair walk takes scenes without meshes too.
     bool packed = true, flat = true;
     for (const auto& st : b->stores) {
-        packed = packed && (st->scene.use_pairs == 3 || st->scene.flat);
-        flat = flat && st->scene.flat;
+        packed = packed && st->scene.walk != 0;
+        flat = flat && st->scene.walk == 7;
     }
     c.walk = flat ? 7 : packed ? 6 : 0;
     b->ctx_shadow = c;

@@ -36,7 +36,9 @@ struct DevScene {
                             // 2: the same, and no leaf is empty (the compact pair walk's condition);
                             // 3: the same, and no tree is deeper than DFPT_WALK_DEPTH (the packed pair
                             // walk's condition)
-    int flat;               // no primitive is a mesh
+    int flat;               // no primitive is a mesh or a terrain
+    int terrain;            // some primitive is a terrain
+    int walk;               // what its rays may walk with when nothing is counted (LaunchCtx::walk)
     const int4* prim_walk;  // {shape type, shape offset, record index, first primitive of the run with this matrix}
     int pair_stack;         // entries of the compact pair walk's stack in use (1..8; 8 unless a test lowers it)
     const float4* shade_tris;  // per triangle (triangle offset / 12), the values surface() reads, copied from

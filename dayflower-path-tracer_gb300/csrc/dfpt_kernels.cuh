@@ -530,12 +530,14 @@ __device__ __forceinline__ void warp_add_stats(const DevParams& P, unsigned long
 // they diverge, and the launch lasts as long as its slowest warp. 8 one-pass frames of instances_scene at
 // 1279 x 717, whose late bounces hold a few thousand rays: closest hits 4.9 -> 3.2 ms, final any-hit
 // 0.82 -> 0.36; 19 passes of mesh_scene at 641 x 479: closest 4.0 -> 3.2, shadow rays 3.1 -> 1.9.
-__device__ __forceinline__ int entries_per_warp(int n) {
+// Terrain marches take much the same time in every lane: their launches fill the warps.
+__device__ __forceinline__ int entries_per_warp(int n, bool terrain) {
+    if (terrain) return 32;
     const int warps = (int)(gridDim.x * (blockDim.x >> 5));
     return min(32, max(1, (n + warps - 1) / warps));
 }
-#define WARP_DYNAMIC(i, n, counter)                                                            \
-    for (int i##_per = entries_per_warp(n), i##_base = 0;;)                                    \
+#define WARP_DYNAMIC(i, n, terrain, counter)                                                   \
+    for (int i##_per = entries_per_warp(n, terrain), i##_base = 0;;)                           \
         if ((i##_base = __shfl_sync(0xFFFFFFFFu, (threadIdx.x & 31) == 0 ? atomicAdd((counter), i##_per) : 0, 0)) >= (n)) break; \
         else for (int i = (int)(threadIdx.x & 31) < i##_per ? i##_base + (int)(threadIdx.x & 31) : (n), i##_once = 1; i##_once; i##_once = 0)
 
@@ -838,7 +840,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(DevScene S0, const DevPar
             __stcs(B.q_hit + i, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset));
         }
     } else {
-        WARP_DYNAMIC(i, n, B.counts + DFPT_COUNTS_FETCH + bounce) {
+        WARP_DYNAMIC(i, n, S0.terrain, B.counts + DFPT_COUNTS_FETCH + bounce) {
             TraceStats st{0, 0};
             const bool valid = i < n;
             float4 o = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 1, 0);
@@ -1255,7 +1257,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow(DevScene S0, const DevPa
             if (h.t >= INF - 0.0001f) unoccluded(i, o, __ldcs(B.s_c + i));
         }
     } else {
-        WARP_DYNAMIC(i, n, B.counts + DFPT_COUNTS_FETCH + DFPT_MAX_DEPTH + 1) {
+        WARP_DYNAMIC(i, n, S0.terrain, B.counts + DFPT_COUNTS_FETCH + DFPT_MAX_DEPTH + 1) {
             TraceStats st{0, 0};
             const bool valid = i < n;
             float4 o = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 1, 0);
@@ -1311,7 +1313,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_final(DevScene S0, const DevPar
             if (!(h.t < INF)) escaped(o, d);
         }
     } else {
-        WARP_DYNAMIC(i, n, B.counts + DFPT_COUNTS_FETCH + bounce) {
+        WARP_DYNAMIC(i, n, S0.terrain, B.counts + DFPT_COUNTS_FETCH + bounce) {
             TraceStats st{0, 0};
             const bool valid = i < n;
             float4 o = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 1, 0);
@@ -1345,7 +1347,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
     const DevBatch Q{};
     int* const fetch = B.counts + DFPT_COUNTS_FETCH + b0;
     const int lane = threadIdx.x & 31;
-    const bool works = lane < entries_per_warp(n);  // few paths are spread over the warps (WARP_DYNAMIC)
+    const bool works = lane < entries_per_warp(n, S.terrain);  // few paths are spread over the warps (WARP_DYNAMIC)
     bool have = false;      // the lane holds a path: its ray waits at bounce b (b == nb: the final any-hit)
     bool drained = false;   // warp-uniform: the queue has no more paths
     int b = nb;
@@ -1494,7 +1496,7 @@ __global__ void __launch_bounds__(128, WALK ? 8 : 1) k_simple(const __grid_const
     // Warps take tiles from the work counter: neighbouring rays walk together, and a warp that drew short
     // ones goes on. Rows in a fixed stride: 1.05 ms for the 1080p ray-cast view of mesh_scene, now 0.80;
     // ambient occlusion at 1003 x 601 0.41, now 0.36.
-    WARP_DYNAMIC(place, n, B.counts + DFPT_COUNTS_FETCH) {
+    WARP_DYNAMIC(place, n, S.terrain, B.counts + DFPT_COUNTS_FETCH) {
         TraceStats st{0, 0};
         uint32_t segs = 0;
         if (place < n) {
