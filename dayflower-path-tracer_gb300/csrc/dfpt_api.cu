@@ -713,14 +713,16 @@ void mark(dfpt_handle* h, int kind) {
     h->events_used++;
 }
 
-// The walk of the launches (LaunchCtx::walk): the counting walks while counting, with a set stack depth and
-// where many primitives of a scene without meshes are looped over because culling is off (its walk is made
-// for the culling BVH; 257 spheres at 640 x 360, culling off: the ray tracer's view 0.38 ms, with that walk
-// 0.46, 8 passes 6.04 and 6.19).
+// The walk of the launches (LaunchCtx::walk): the counting walks while counting, with a set stack depth, for
+// the ray marcher (it traces no rays, and that kernel takes rows) and where many primitives of a scene without
+// meshes are looped over because culling is off (its walk is made for the culling BVH; 257 spheres at
+// 640 x 360, culling off: the ray tracer's view 0.38 ms, with that walk 0.46, 8 passes 6.04 and 6.19).
 void refresh_walk(dfpt_handle* h) {
     const DevScene& S = h->sc.scene;
+    const int rt = h->params.renderer_type;
     const bool loop = S.walk == 7 && h->sc.culling_available && S.use_culling == 0;
-    const int walk = h->counting || loop || (S.walk == 6 && S.pair_stack != 8) ? 0 : S.walk;
+    const int walk = h->counting || rt == DFPT_RENDERER_RAY_MARCHER || loop || (S.walk == 6 && S.pair_stack != 8) ? 0 : S.walk;
+    h->ctx.one_ray = rt == DFPT_RENDERER_SURFACE_NORMALS;
     if (walk == h->ctx.walk) return;
     h->ctx.walk = walk;
     h->graph_valid = false;

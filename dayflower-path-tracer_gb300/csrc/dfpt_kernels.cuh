@@ -541,6 +541,12 @@ __device__ __forceinline__ int entries_per_warp(int n, bool terrain) {
         if ((i##_base = __shfl_sync(0xFFFFFFFFu, (threadIdx.x & 31) == 0 ? atomicAdd((counter), i##_per) : 0, 0)) >= (n)) break; \
         else for (int i = (int)(threadIdx.x & 31) < i##_per ? i##_base + (int)(threadIdx.x & 31) : (n), i##_once = 1; i##_once; i##_once = 0)
 
+// The next 32 places past the first `taken`, which went by warp; n when there are none. All lanes call it.
+__device__ __forceinline__ int next_pixels(int n, int taken, int* counter) {
+    if (n <= taken) return n;
+    return taken + __shfl_sync(0xFFFFFFFFu, (threadIdx.x & 31) == 0 ? atomicAdd(counter, 32) : 0, 0);
+}
+
 #define GRID_STRIDE_UNIFORM(i, n)                                                              \
     for (int i##_base = blockIdx.x * blockDim.x; i##_base < (n); i##_base += gridDim.x * blockDim.x) \
         for (int i = i##_base + (int)threadIdx.x, i##_once = 1; i##_once; i##_once = 0)
@@ -1427,23 +1433,23 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tail(DevScene S, const DevParam
 // ---------------------------------------------------------------------------------------------
 // The per-pixel modes: ray caster, ambient occlusion, surface normals, ray tracer, ray marcher.
 
-// WALK 6 and 7: the packed pair walk or the walk of scenes without meshes for every ray (LaunchCtx::walk;
-// nothing is counted), in a function of its own: k_simple calls it from four places and needs few
-// registers beside it (64 against 112, 8 blocks of 128 per SM against 4: the 1080p ray-cast view of
-// mesh_scene 1.80 -> 1.31 ms, ambient occlusion at 1003 x 601 0.71 -> 0.50 ms with its readbacks).
-template <int WALK>
+// k_simple<WALK, MINB>. WALK 6 and 7: the packed pair walk or the walk of scenes without meshes for every ray
+// (LaunchCtx::walk; nothing is counted). The packed walk is a function of its own: k_simple calls it from four
+// places and needs few registers beside it (in place and uncapped 131; the 1080p ray-cast view of mesh_scene
+// 1.80 -> 1.31 ms, ambient occlusion at 1003 x 601 0.71 -> 0.50 with its readbacks).
+template <int MINB>
 __device__ __noinline__ Hit trace_simple_walk(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz) {
-    if constexpr (WALK == 7) return trace_flat<false>(S, ox, oy, oz, dx, dy, dz);
-    else return trace_pairs<false, 128>(S, ox, oy, oz, dx, dy, dz);
+    return trace_pairs<false, 128>(S, ox, oy, oz, dx, dy, dz);
 }
-template <int WALK>
+template <int WALK, int MINB>
 __device__ __forceinline__ Hit trace_simple(const DevScene& S, float ox, float oy, float oz, float dx, float dy, float dz, TraceStats& st) {
-    if constexpr (WALK != 0) return trace_simple_walk<WALK>(S, ox, oy, oz, dx, dy, dz);
+    if constexpr (WALK == 7) return trace_flat<false>(S, ox, oy, oz, dx, dy, dz);
+    else if constexpr (WALK == 6) return trace_simple_walk<MINB>(S, ox, oy, oz, dx, dy, dz);
     else return trace_s(S, ox, oy, oz, dx, dy, dz, st);
 }
 
 // doShaderPhongReflectionModel0 (GRK:1962-2039), with the reference's closest-hit shadow test.
-template <int WALK>
+template <int WALK, int MINB>
 __device__ int phong0(const DevScene& S, const DevParams& P, bool test, float px, float py, float pz, float nx, float ny, float nz,
                       float vx, float vy, float vz, float ar, float ag, float ab, TraceStats& st) {
     float r = 0.0f, g = 0.0f, b = 0.0f;
@@ -1454,7 +1460,7 @@ __device__ int phong0(const DevScene& S, const DevParams& P, bool test, float px
     const float lr = 1.0f / ll;
     const float lnx = lx * lr, lny = ly * lr, lnz = lz * lr;
     float t = INF;
-    if (test) t = trace_simple<WALK>(S, px, py, pz, lnx, lny, lnz, st).t;
+    if (test) t = trace_simple<WALK, MINB>(S, px, py, pz, lnx, lny, lnz, st).t;
     if (t >= INF || t > l2) {
         const float ldn = lnx * nx + lny * ny + lnz * nz;
         r += ar * 0.5f * jmax(ldn, 0.0f) * 1.0f;
@@ -1487,20 +1493,27 @@ __device__ float height_rm(const DevParams& P, float x, float z) {
     return fractal2(P.g_amplitude, P.g_frequency, P.g_gain, P.g_lacunarity, P.g_octaves, x, z);
 }
 
-template <int WALK>
-__global__ void __launch_bounds__(128, WALK ? 8 : 1) k_simple(const __grid_constant__ DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
+template <int WALK, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_simple(const __grid_constant__ DevScene S, const DevParams* __restrict__ Pp, DevPass B) {
     const DevParams& P = *Pp;
     const int n = B.n_pixels;
     const uint32_t pass = (uint32_t)*B.pass_index;
     const int mode = P.renderer_type;
-    // Warps take tiles from the work counter: neighbouring rays walk together, and a warp that drew short
-    // ones goes on. Rows in a fixed stride: 1.05 ms for the 1080p ray-cast view of mesh_scene, now 0.80;
-    // ambient occlusion at 1003 x 601 0.41, now 0.36.
-    WARP_DYNAMIC(place, n, S.terrain, B.counts + DFPT_COUNTS_FETCH) {
+    // A warp takes 32 pixels at a time, the first by its place in the grid, more from the work counter: the
+    // packed walks a tile, so that neighbouring rays walk together (rows in a fixed stride: 1.05 ms for the
+    // 1080p ray-cast view of mesh_scene, tiles 0.80); the counting walk, which also serves the ray marcher and
+    // scenes with terrains, a piece of a row: marches of one row are much the same length (a terrain at
+    // 320 x 240 in tiles 0.32 ms, in rows 0.17; the marcher 1.40 and 0.73). Frames of fewer pixels than the
+    // launch has lanes take full warps and leave the others idle: half-filled warps repeat the shading
+    // (noise normal maps at 320 x 240: 0.087 ms with 16 pixels a warp, 0.040 with 32).
+    const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * (blockDim.x >> 5));
+    for (int first = 32 * (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); first < n;
+         first = next_pixels(n, 32 * warps, B.counts + DFPT_COUNTS_FETCH)) {
+        const int place = first + lane;
         TraceStats st{0, 0};
         uint32_t segs = 0;
         if (place < n) {
-            const int i = pixel_at(P.width, P.height, place);
+            const int i = WALK == 0 ? place : pixel_at(P.width, P.height, place);
             Rng rng = make_rng(P, (uint32_t)i, pass, P.rng_kind == DFPT_RNG_LCG ? B.rng[i] : 0ull);
             float4 o4, d4;
             const bool live = primary_ray(S, P, i, false, rng, o4, d4);
@@ -1527,7 +1540,7 @@ __global__ void __launch_bounds__(128, WALK ? 8 : 1) k_simple(const __grid_const
                             const float nr = 1.0f / sqrtf(nx * nx + ny * ny + nz * nz);
                             const float noise = fbm3(8.0f, 0.5f, 0.0f, 1.0f, 16, px, py, pz);
                             const float al = saturate_j(noise * 1.0f + 0.1f, 0.0f, 1.0f);
-                            const int c = phong0<WALK>(S, P, false, px, py, pz, nx * nr, ny * nr, nz * nr, -dx, -dy, -dz, al, al, al, st);
+                            const int c = phong0<WALK, MINB>(S, P, false, px, py, pz, nx * nr, ny * nr, nz * nr, -dx, -dy, -dz, al, al, al, st);
                             cr_ = cr(c); cg_ = cg(c); cb_ = cb(c);
                             t = max_t;
                         }
@@ -1536,7 +1549,7 @@ __global__ void __launch_bounds__(128, WALK ? 8 : 1) k_simple(const __grid_const
                 } else {
                     const int depth_max = mode == DFPT_RENDERER_RAY_TRACER ? 5 : 1;
                     for (int depth = 0; depth < depth_max; ++depth) {
-                        const Hit h = trace_simple<WALK>(S, ox, oy, oz, dx, dy, dz, st);
+                        const Hit h = trace_simple<WALK, MINB>(S, ox, oy, oz, dx, dy, dz, st);
                         segs++;
                         if (depth == 0) B.primitive_offsets[i] = h.prim >= 0 ? h.prim * 3 : -1;
                         if (h.t == INF || h.prim == -1) {
@@ -1575,7 +1588,7 @@ __global__ void __launch_bounds__(128, WALK ? 8 : 1) k_simple(const __grid_const
                             const float e1z = e0x * u2z + e0y * v0z + e0z * w1z;
                             const float er = rsqrt_j(e1x * e1x + e1y * e1y + e1z * e1z);
                             const float aox = s.px + w1x * 0.01f, aoy = s.py + w1y * 0.01f, aoz = s.pz + w1z * 0.01f;
-                            const float t = trace_simple<WALK>(S, aox, aoy, aoz, e1x * er, e1y * er, e1z * er, st).t;
+                            const float t = trace_simple<WALK, MINB>(S, aox, aoy, aoz, e1x * er, e1y * er, e1z * er, st).t;
                             segs++;
                             const bool hit = t < P.ao_max_distance;
                             const float v = hit ? 1.0f : 0.0f;  // bright 1, dark 0
@@ -1592,7 +1605,7 @@ __global__ void __launch_bounds__(128, WALK ? 8 : 1) k_simple(const __grid_const
                         } else {
                             ar = cr(albedo); ag = cg(albedo); ab = cb(albedo);
                         }
-                        const int c = phong0<WALK>(S, P, true, s.px, s.py, s.pz, wx, wy, wz, -dx, -dy, -dz, ar, ag, ab, st);
+                        const int c = phong0<WALK, MINB>(S, P, true, s.px, s.py, s.pz, wx, wy, wz, -dx, -dy, -dz, ar, ag, ab, st);
                         segs++;
                         if (mode == DFPT_RENDERER_RAY_CASTER) {
                             cr_ = cr(c); cg_ = cg(c); cb_ = cb(c);
@@ -2439,10 +2452,21 @@ static void launch_diff_reduce(const LaunchCtx& c, const double* rows, int n_row
 }
 #endif
 #ifndef DFPT_ONE_SCENE
+// Resident blocks, by what a view's time goes on. The packed walk at 8 (64 registers, 0.6 KB of spills) hides its
+// waits behind other warps (a ray-cast view of mesh_scene with 112,000 triangles at 1280 x 720: 0.37 ms, at 4
+// 0.40); where every warp has one tile (frames up to 4 blocks' lanes) or one ray a pixel (surface normals)
+// those warps are few or soon done, and 4 blocks without spills win: 180 triangles at 320 x 240, four views
+// 4-10 % faster, surface normals of 36 triangles at 1280 x 720 0.084 -> 0.078 ms. Scenes without meshes 6: 4
+// is 3-8 % slower at 1280 x 720, 8 10 % in small views. The counting walk 6, the registers it takes uncapped.
 static void launch_simple(const LaunchCtx& c) {
-    if (c.walk == 6) k_simple<6><<<resident_grid(k_simple<6>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
-    else if (c.walk == 7) k_simple<7><<<resident_grid(k_simple<7>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
-    else k_simple<0><<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    if (c.walk == 0) {
+        k_simple<0, 6><<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+        return;
+    }
+    const int roomy = c.walk == 7 ? resident_grid(k_simple<7, 6>, 128) : resident_grid(k_simple<6, 4>, 128);
+    if (c.walk == 7) k_simple<7, 6><<<roomy, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    else if (c.one_ray || c.pass->n_pixels <= roomy * 128) k_simple<6, 4><<<roomy, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    else k_simple<6, 8><<<resident_grid(k_simple<6, 8>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
 }
 static void launch_wireframe(const LaunchCtx& c) { k_wireframe<<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass); }
 static void launch_film(const LaunchCtx& c) { k_film<<<full_grid<k_film>(256), 256, 0, c.stream>>>(c.params, *c.pass); }
@@ -2476,7 +2500,7 @@ static void occupancy(int sms, int& grid, int& grid_trace, int& grid_simple) {
     b3 = b1;
 #else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_shade<false>, 256, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, k_simple<0>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, k_simple<0, 6>, 128, 0);
 #endif
     grid = sms * (b1 > 0 ? b1 : 1);
     grid_trace = trace_grid(0, sms);
