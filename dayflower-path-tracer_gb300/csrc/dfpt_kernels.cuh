@@ -2161,29 +2161,23 @@ __global__ void k_init_tables(const int* perm256, const float* grad36) {
 // Resident blocks of 256 for scenes without meshes: 4 (48-56 registers, no spills); 5, 6 and 8 measured
 // 0.46, 0.50 and 0.76 ms against 0.44 for the closest hits of 64 passes of sphere_scene.
 #define DFPT_FLAT_MINB 4
-// A grid of every block of a kernel that the device holds at once, found once per process. Camera and film
-// ran on k_shade's grid, 3 blocks of 256 per SM, where 5 and 8 fit: 8 frames at 1080p 0.34 -> 0.31 and 0.60
-// -> 0.41 ms. The binning's scatters stay on that grid: with 8 blocks 3.58 -> 3.82 ms of a 32-pass still,
-// their writes spread over more bins at a time.
-template <auto Kernel>
-static int full_grid(int block) {
-    static const int grid = [](int block) {
-        int dev = 0, sms = 0, b = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, Kernel, block, 0);
-        return (sms > 0 ? sms : 1) * (b > 0 ? b : 1);
-    }(block);
-    return grid;
-}
-// A grid of every block of `kernel` that the current device holds at once.
+// A grid of every block of a kernel that the device holds at once.
 template <class Kernel>
-static int resident_grid(Kernel kernel, int block, size_t dynamic_shared = 0) {
+static int device_grid(Kernel kernel, int block, size_t dynamic_shared) {
     int dev = 0, sms = 0, b = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, block, dynamic_shared);
     return (sms > 0 ? sms : 1) * (b > 0 ? b : 1);
+}
+// The same for a kernel without dynamic shared memory, found once per process: the replay of a differentiable
+// render launches directly, several kernels a bounce. Camera and film ran on k_shade's grid, 3 blocks of 256 per
+// SM, where 5 and 8 fit: 8 frames at 1080p 0.34 -> 0.31 and 0.60 -> 0.41 ms. The binning's scatters stay on
+// that grid: with 8 blocks 3.58 -> 3.82 ms of a 32-pass still, their writes spread over more bins at a time.
+template <auto Kernel, int Block>
+static int full_grid() {
+    static const int grid = device_grid(Kernel, Block, 0);
+    return grid;
 }
 
 template <int V, int BLOCK, int MINB>
@@ -2203,11 +2197,11 @@ struct TraceCfg {
     static void closest(const LaunchCtx& c, int bounce) {
         if constexpr (V == 5) {
             if (c.walk == 6) {
-                k_trace<false, false, 6, BLOCK, MINB><<<resident_grid(k_trace<false, false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                k_trace<false, false, 6, BLOCK, MINB><<<full_grid<k_trace<false, false, 6, BLOCK, MINB>, BLOCK>(), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
                 return;
             }
             if (c.walk == 7) {
-                k_trace<false, false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_trace<false, false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                k_trace<false, false, 7, 256, DFPT_FLAT_MINB><<<full_grid<k_trace<false, false, 7, 256, DFPT_FLAT_MINB>, 256>(), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
                 return;
             }
         }
@@ -2216,11 +2210,11 @@ struct TraceCfg {
     static void shadow(const LaunchCtx& c, int bounce) {
         if constexpr (V == 5) {
             if (c.walk == 6) {
-                k_shadow<false, 6, BLOCK, MINB><<<resident_grid(k_shadow<false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                k_shadow<false, 6, BLOCK, MINB><<<full_grid<k_shadow<false, 6, BLOCK, MINB>, BLOCK>(), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
                 return;
             }
             if (c.walk == 7) {
-                k_shadow<false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_shadow<false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                k_shadow<false, 7, 256, DFPT_FLAT_MINB><<<full_grid<k_shadow<false, 7, 256, DFPT_FLAT_MINB>, 256>(), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
                 return;
             }
         }
@@ -2229,11 +2223,11 @@ struct TraceCfg {
     static void final_(const LaunchCtx& c, int bounce) {
         if constexpr (V == 5) {
             if (c.walk == 6) {
-                k_final<false, 6, BLOCK, MINB><<<resident_grid(k_final<false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                k_final<false, 6, BLOCK, MINB><<<full_grid<k_final<false, 6, BLOCK, MINB>, BLOCK>(), BLOCK, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
                 return;
             }
             if (c.walk == 7) {
-                k_final<false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_final<false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
+                k_final<false, 7, 256, DFPT_FLAT_MINB><<<full_grid<k_final<false, 7, 256, DFPT_FLAT_MINB>, 256>(), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce);
                 return;
             }
         }
@@ -2254,15 +2248,15 @@ struct TraceCfg {
     static void tail_t(const LaunchCtx& c, int b0, int nb) {
         if constexpr (TVV == 5) {
             if (c.walk == 6) {
-                k_tail<6, 256, TB><<<resident_grid(k_tail<6, 256, TB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
+                k_tail<6, 256, TB><<<full_grid<k_tail<6, 256, TB>, 256>(), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
                 return;
             }
             if (c.walk == 7) {
-                k_tail<7, 256, TB><<<resident_grid(k_tail<7, 256, TB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
+                k_tail<7, 256, TB><<<full_grid<k_tail<7, 256, TB>, 256>(), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
                 return;
             }
         }
-        k_tail<TVV, 256, TB><<<resident_grid(k_tail<TVV, 256, TB>, 256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
+        k_tail<TVV, 256, TB><<<full_grid<k_tail<TVV, 256, TB>, 256>(), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, b0, nb);
     }
     static void tail(const LaunchCtx& c, int b0, int nb) {
 #ifdef DFPT_EXTENDED_KERNELS
@@ -2280,11 +2274,11 @@ struct TraceCfg {
     static void b_closest(const LaunchCtx& c, int bounce) {
         if constexpr (BV == 5) {
             if (c.walk == 6) {
-                k_trace<true, false, 6, BLOCK, MINB><<<resident_grid(k_trace<true, false, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                k_trace<true, false, 6, BLOCK, MINB><<<full_grid<k_trace<true, false, 6, BLOCK, MINB>, BLOCK>(), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
                 return;
             }
             if (c.walk == 7) {
-                k_trace<true, false, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_trace<true, false, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
+                k_trace<true, false, 7, 256, DFPT_FLAT_MINB><<<full_grid<k_trace<true, false, 7, 256, DFPT_FLAT_MINB>, 256>(), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce, c.pass->sorted_queues ? 0 : (bounce & 1));
                 return;
             }
         }
@@ -2293,11 +2287,11 @@ struct TraceCfg {
     static void b_shadow(const LaunchCtx& c, int bounce) {
         if constexpr (BV == 5) {
             if (c.walk == 6) {
-                k_shadow<true, 6, BLOCK, MINB><<<resident_grid(k_shadow<true, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                k_shadow<true, 6, BLOCK, MINB><<<full_grid<k_shadow<true, 6, BLOCK, MINB>, BLOCK>(), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
                 return;
             }
             if (c.walk == 7) {
-                k_shadow<true, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_shadow<true, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                k_shadow<true, 7, 256, DFPT_FLAT_MINB><<<full_grid<k_shadow<true, 7, 256, DFPT_FLAT_MINB>, 256>(), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
                 return;
             }
         }
@@ -2306,11 +2300,11 @@ struct TraceCfg {
     static void b_final(const LaunchCtx& c, int bounce) {
         if constexpr (BV == 5) {
             if (c.walk == 6) {
-                k_final<true, 6, BLOCK, MINB><<<resident_grid(k_final<true, 6, BLOCK, MINB>, BLOCK), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                k_final<true, 6, BLOCK, MINB><<<full_grid<k_final<true, 6, BLOCK, MINB>, BLOCK>(), BLOCK, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
                 return;
             }
             if (c.walk == 7) {
-                k_final<true, 7, 256, DFPT_FLAT_MINB><<<resident_grid(k_final<true, 7, 256, DFPT_FLAT_MINB>, 256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
+                k_final<true, 7, 256, DFPT_FLAT_MINB><<<full_grid<k_final<true, 7, 256, DFPT_FLAT_MINB>, 256>(), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce);
                 return;
             }
         }
@@ -2378,7 +2372,7 @@ static int trace_grid(int config, int sms) {
 }
 
 #ifndef DFPT_ONE_SCENE
-static void launch_camera(const LaunchCtx& c) { k_camera<false><<<full_grid<k_camera<false>>(256), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}); }
+static void launch_camera(const LaunchCtx& c) { k_camera<false><<<full_grid<k_camera<false>, 256>(), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}); }
 static void launch_shade(const LaunchCtx& c, int bounce) { k_shade<false><<<c.grid, 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, DevBatch{}, bounce); }
 #endif
 
@@ -2400,11 +2394,11 @@ BATCH_DISPATCH(final)
 #undef BATCH_CASE_closest
 #undef BATCH_CASE_shadow
 #undef BATCH_CASE_final
-static void launch_b_camera(const LaunchCtx& c, int) { k_camera<true><<<full_grid<k_camera<true>>(256), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch); }
+static void launch_b_camera(const LaunchCtx& c, int) { k_camera<true><<<full_grid<k_camera<true>, 256>(), 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch); }
 static void launch_b_shade(const LaunchCtx& c, int bounce) { k_shade<true><<<c.grid, 256, 0, c.stream>>>(BATCH_SCENE(c), c.params, *c.pass, *c.batch, bounce); }
 static void launch_b_wave(const LaunchCtx& c, int) { k_bwave<<<1, 32, 0, c.stream>>>(*c.batch); }
-static void launch_b_film(const LaunchCtx& c, int) { k_bfilm<<<full_grid<k_bfilm>(256), 256, 0, c.stream>>>(*c.batch, *c.pass); }
-static void launch_b_resolve(const LaunchCtx& c, int) { k_bresolve<<<full_grid<k_bresolve>(256), 256, 0, c.stream>>>(*c.batch, *c.pass); }
+static void launch_b_film(const LaunchCtx& c, int) { k_bfilm<<<full_grid<k_bfilm, 256>(), 256, 0, c.stream>>>(*c.batch, *c.pass); }
+static void launch_b_resolve(const LaunchCtx& c, int) { k_bresolve<<<full_grid<k_bresolve, 256>(), 256, 0, c.stream>>>(*c.batch, *c.pass); }
 static void launch_b_end(const LaunchCtx& c, int) { k_bend_wave<<<1, 32, 0, c.stream>>>(*c.batch); }
 static void launch_b_shadow_reset(const LaunchCtx& c, int) { k_shadow_reset<<<1, 32, 0, c.stream>>>(*c.pass); }
 // Bins the rays shading queued for bounce + 1 (queue 1 -> queue 0). k_shade counts the bins as it
@@ -2432,8 +2426,8 @@ static void launch_shade_adj_t(const LaunchCtx& c, int bounce) {
     // A row per block; no more blocks than are resident (at 128 registers 2 per SM, where c.grid's 3 left a
     // second round half empty).
     const int rows = c.pass->diff_row_count;
-    if (bytes <= 44 * 1024) k_shade_adj<BATCH, true><<<std::min(rows, resident_grid(k_shade_adj<BATCH, true>, 256, bytes)), 256, bytes, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
-    else k_shade_adj<BATCH, false><<<std::min(rows, resident_grid(k_shade_adj<BATCH, false>, 256)), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
+    if (bytes <= 44 * 1024) k_shade_adj<BATCH, true><<<std::min(rows, device_grid(k_shade_adj<BATCH, true>, 256, bytes)), 256, bytes, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
+    else k_shade_adj<BATCH, false><<<std::min(rows, full_grid<k_shade_adj<BATCH, false>, 256>()), 256, 0, c.stream>>>(*c.scene, c.params, *c.pass, Q, bounce);
 }
 template <bool BATCH>
 static void launch_final_adj_t(const LaunchCtx& c, int bounce) {
@@ -2463,13 +2457,13 @@ static void launch_simple(const LaunchCtx& c) {
         k_simple<0, 6><<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
         return;
     }
-    const int roomy = c.walk == 7 ? resident_grid(k_simple<7, 6>, 128) : resident_grid(k_simple<6, 4>, 128);
-    if (c.walk == 7) k_simple<7, 6><<<roomy, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    const int roomy = full_grid<k_simple<6, 4>, 128>();
+    if (c.walk == 7) k_simple<7, 6><<<full_grid<k_simple<7, 6>, 128>(), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
     else if (c.one_ray || c.pass->n_pixels <= roomy * 128) k_simple<6, 4><<<roomy, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
-    else k_simple<6, 8><<<resident_grid(k_simple<6, 8>, 128), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
+    else k_simple<6, 8><<<full_grid<k_simple<6, 8>, 128>(), 128, 0, c.stream>>>(*c.scene, c.params, *c.pass);
 }
 static void launch_wireframe(const LaunchCtx& c) { k_wireframe<<<c.grid_simple, 128, 0, c.stream>>>(*c.scene, c.params, *c.pass); }
-static void launch_film(const LaunchCtx& c) { k_film<<<full_grid<k_film>(256), 256, 0, c.stream>>>(c.params, *c.pass); }
+static void launch_film(const LaunchCtx& c) { k_film<<<full_grid<k_film, 256>(), 256, 0, c.stream>>>(c.params, *c.pass); }
 static void launch_end_pass(const LaunchCtx& c) { k_end_pass<<<1, 32, 0, c.stream>>>(*c.pass); }
 // Bins a plain pass's deferred shadow rays into `to` (a pass record whose s_* point at the second
 // set); shading counted the bins. Returns the kernels launched.
@@ -2486,9 +2480,9 @@ static int launch_sort_rays(const LaunchCtx& c, int bounce, const DevPass& to) {
     k_sort_rays_scatter_plain<<<c.grid, 256, 0, c.stream>>>(*c.scene, *c.pass, bounce, to.q_o[qi], to.q_d[qi]);
     return k + 1;
 }
-static void launch_film_mean(const LaunchCtx& c, double* out3) { k_film_mean<<<full_grid<k_film_mean>(256), 256, 0, c.stream>>>(*c.pass, out3); }
+static void launch_film_mean(const LaunchCtx& c, double* out3) { k_film_mean<<<full_grid<k_film_mean, 256>(), 256, 0, c.stream>>>(*c.pass, out3); }
 static void launch_film_average(const LaunchCtx& c, float* rgb, int* samples) {
-    k_film_average<<<full_grid<k_film_average>(256), 256, 0, c.stream>>>(*c.pass, rgb, samples);
+    k_film_average<<<full_grid<k_film_average, 256>(), 256, 0, c.stream>>>(*c.pass, rgb, samples);
 }
 #endif
 static void launch_init_tables(cudaStream_t s, const int* perm, const float* grad) { k_init_tables<<<1, 512, 0, s>>>(perm, grad); }
