@@ -50,7 +50,7 @@ METRIC = "M path samples/s @1080p"
 UNIT = "M samples/s"
 # Measured DRAM bytes (read + write) per closest-hit segment of the traversal kernel on
 # mesh_scene: one ncu capture of the traversal kernel at 960x540.
-TRACE_DRAM_BYTES_PER_SEGMENT = 65.5
+TRACE_DRAM_BYTES_PER_SEGMENT = 60.8
 
 
 def parse():
@@ -553,8 +553,8 @@ def frame_kernels(k, frames=8):
 # slots, configuration 17, the packed pair walk; bounces 0 and 1): active lanes per issued instruction,
 # the fraction of cycles with an instruction issued, and warps active (of the SM's maximum; the register
 # limit allows 0.625).
-TRACE_NCU = {"config": 17, "lanes_per_instruction": {"bounce0": 19.7, "bounce1": 10.7}, "issue_active": [0.645, 0.591],
-             "warps_active": [0.596, 0.544]}
+TRACE_NCU = {"config": 17, "lanes_per_instruction": {"bounce0": 16.9, "bounce1": 9.4}, "issue_active": [0.623, 0.571],
+             "warps_active": [0.571, 0.522]}
 
 
 def main():
@@ -752,11 +752,10 @@ def main():
     hbm = hbm or 6800.0
     closest_segments = cnt[0]
     # Visits per closest-hit segment, the timed kernel's work: the GPU's own counters over a step.
-    # Counting walks visit nodes in the reference's order: without primitive culling the counts equal
-    # the reference algorithm's (the CPU restatement's on its sample are reported beside them), with
-    # culling they leave out the primitives the GPU skips. The timed walk counts nothing and enters
-    # the nearer child first where the order cannot matter, so it visits somewhat fewer nodes than
-    # these algorithmic ones (camera rays of mesh_scene: 42 of 52 box tests).
+    # Without primitive culling the counts equal the reference algorithm's (the CPU restatement's on
+    # its sample are reported beside them), with culling they leave out the primitives the GPU skips.
+    # The timed walk counts nothing, but tests the same boxes and triangles in the same order, two
+    # boxes to a 64-byte record.
     nodes_per_seg = cnt[4] / max(cnt[0], 1)
     tris_per_seg = cnt[5] / max(cnt[0], 1)
     bytes_per_seg = nodes_per_seg * 32 + tris_per_seg * 48 + 64
@@ -814,8 +813,8 @@ def main():
                                     "(dfpt_probe_read_bandwidth, best of 24/48/64 MiB buffers)",
                      "peak_by_buffer_mib": l2_sizes,
                      "kernel": "k_trace<closest>", "avg_launch_ms": avg_trace_ms,
-                     "note": "algorithmic bytes = node and triangle records the reference-order walk visits per closest-hit segment "
-                             "(the timed walk, nearer child first, visits fewer); the records are "
+                     "note": "algorithmic bytes = boxes (32 B) and triangles (48 B) tested per closest-hit segment, each lane's counted (lanes of "
+                             "a warp on one record share its load); the records are "
                              "L2-resident, so the roof is L2 read bandwidth; DRAM carries the rays (traffic)",
                      "hbm": {"peak": hbm, "peak_source": hbm_note, "dram_gbs": dram_gbs,
                              "dram_frac": dram_gbs / hbm if dram_gbs else None,
