@@ -45,7 +45,8 @@ __device__ int image_texture_simple(const float* S, int to, float u, float v) {
     return index >= 0 && index < res ? f2i(texf(S, to + 8 + index)) : 0;
 }
 
-__device__ __noinline__ Surf terrain_surface(float oxo, float oyo, float ozo, float dxo, float dyo, float dzo, float t) {
+// Inlined: as a function of its own the compiler fused other products, and paths went another way.
+__device__ __forceinline__ Surf terrain_surface(float oxo, float oyo, float ozo, float dxo, float dyo, float dzo, float t) {
     Surf s;
     s.tx = s.ty = s.tz = 0.0f;
     const float sr = 1.0f / 10.0f;
