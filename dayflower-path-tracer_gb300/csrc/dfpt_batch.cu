@@ -217,12 +217,14 @@ int batch_prepare(dfpt_batch* b) {
     c.trace_config = b->trace_config;
     c.grid_trace = b->ks.trace_grid(b->trace_config, b->sms);
     // One launch walks every scene's rays; the packed pair walk takes scenes without meshes too.
-    bool packed = true, flat = true;
+    bool packed = true, flat = true, terrain = true;
     for (const auto& st : b->stores) {
         packed = packed && st->scene.walk != 0;
         flat = flat && st->scene.walk == 7;
+        terrain = terrain && st->scene.terrain;
     }
     c.walk = flat ? 7 : packed ? 6 : 0;
+    c.terrain = terrain;
     b->ctx_shadow = c;
     b->ctx_shadow.pass = &b->pass_shadow;
     return DFPT_OK;

@@ -20,6 +20,7 @@ struct LaunchCtx {
     // What configurations 16 and 17 and the per-pixel modes walk with: 6 the packed pair walk, 7 scenes
     // without meshes, 0 the configuration's own (counting) walk.
     int walk = 0;
+    bool terrain = false;  // batch launches: every scene has a terrain (entries_per_warp)
     bool one_ray = false;  // the per-pixel mode traces a pixel's camera ray only
 };
 
