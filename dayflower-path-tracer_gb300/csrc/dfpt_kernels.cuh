@@ -538,9 +538,23 @@ __device__ __forceinline__ int entries_per_warp(int n, bool terrain) {
     const int warps = (int)(gridDim.x * (blockDim.x >> 5));
     return min(32, max(1, (n + warps - 1) / warps));
 }
+// A warp's next entries. With terrains the first ones go by place, neighbouring entries to different SMs, and only those
+// past the launch's lanes come from the counter: the long marches of a frame are neighbours, and the warps that reach
+// the counter first sit together on few SMs (one pass at 200 x 150 1.43 -> 0.90 ms, 1.32 before rays were spread at
+// all; at 320 x 240 1.63 -> 1.05, 1.53 before; 641 x 479 2.44 -> 2.11, 2.40). Other walks are shorter and keep the counter.
+__device__ __forceinline__ int next_entries(int n, int per, bool terrain, int& taken, int* counter) {
+    if (terrain) {
+        if (taken == 0) {
+            taken = 32 * (int)(gridDim.x * (blockDim.x >> 5));
+            return 32 * (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+        }
+        if (n <= taken) return n;
+    }
+    return taken + __shfl_sync(0xFFFFFFFFu, (threadIdx.x & 31) == 0 ? atomicAdd(counter, per) : 0, 0);
+}
 #define WARP_DYNAMIC(i, n, terrain, counter)                                                   \
-    for (int i##_per = entries_per_warp(n, terrain), i##_base = 0;;)                           \
-        if ((i##_base = __shfl_sync(0xFFFFFFFFu, (threadIdx.x & 31) == 0 ? atomicAdd((counter), i##_per) : 0, 0)) >= (n)) break; \
+    for (int i##_per = entries_per_warp(n, terrain), i##_taken = 0, i##_base = 0;;)            \
+        if ((i##_base = next_entries(n, i##_per, terrain, i##_taken, counter)) >= (n)) break;  \
         else for (int i = (int)(threadIdx.x & 31) < i##_per ? i##_base + (int)(threadIdx.x & 31) : (n), i##_once = 1; i##_once; i##_once = 0)
 
 // The next 32 places past the first `taken`, which went by warp; n when there are none. All lanes call it.
@@ -848,7 +862,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(DevScene S0, const DevPar
             __stcs(B.q_hit + i, make_int4(__float_as_int(h.t), h.prim, h.shape_type, h.shape_offset));
         }
     } else {
-        WARP_DYNAMIC(i, n, S0.terrain, B.counts + DFPT_COUNTS_FETCH + bounce) {
+        WARP_DYNAMIC(i, n, V < 6 && S0.terrain, B.counts + DFPT_COUNTS_FETCH + bounce) {
             TraceStats st{0, 0};
             const bool valid = i < n;
             float4 o = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 1, 0);
@@ -1265,7 +1279,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_shadow(DevScene S0, const DevPa
             if (h.t >= INF - 0.0001f) unoccluded(i, o, __ldcs(B.s_c + i));
         }
     } else {
-        WARP_DYNAMIC(i, n, S0.terrain, B.counts + DFPT_COUNTS_FETCH + DFPT_MAX_DEPTH + 1) {
+        WARP_DYNAMIC(i, n, V < 6 && S0.terrain, B.counts + DFPT_COUNTS_FETCH + DFPT_MAX_DEPTH + 1) {
             TraceStats st{0, 0};
             const bool valid = i < n;
             float4 o = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 1, 0);
@@ -1321,7 +1335,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_final(DevScene S0, const DevPar
             if (!(h.t < INF)) escaped(o, d);
         }
     } else {
-        WARP_DYNAMIC(i, n, S0.terrain, B.counts + DFPT_COUNTS_FETCH + bounce) {
+        WARP_DYNAMIC(i, n, V < 6 && S0.terrain, B.counts + DFPT_COUNTS_FETCH + bounce) {
             TraceStats st{0, 0};
             const bool valid = i < n;
             float4 o = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 1, 0);
@@ -1503,7 +1517,7 @@ __global__ void __launch_bounds__(128, MINB) k_simple(const __grid_constant__ De
     const int mode = P.renderer_type;
     // A warp takes 32 pixels at a time, the first by its place in the grid, more from the work counter: the
     // packed walks a tile, so that neighbouring rays walk together (rows in a fixed stride: 1.05 ms for the
-    // 1080p ray-cast view of mesh_scene, tiles 0.80); the counting walk, which also serves the ray marcher and
+    // 1080p ray-cast view of mesh_scene, tiles 0.84); the counting walk, which also serves the ray marcher and
     // scenes with terrains, a piece of a row: marches of one row are much the same length (a terrain at
     // 320 x 240 in tiles 0.32 ms, in rows 0.17; the marcher 1.40 and 0.73). Frames of fewer pixels than the
     // launch has lanes take full warps and leave the others idle: half-filled warps repeat the shading
